@@ -764,6 +764,350 @@ __global__ void __launch_bounds__(256) prefilter_tiled_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------
+// FFT form of the pre-filter (order 64 .. 4096, i.e. W <= 2048).  The ramp
+// kernel is as long as the row, so the direct form costs 2 W flops per output
+// (58 GFLOP at 384^2 x 512 views, 2.47 ms); one transform pair costs ~60
+// whatever W is.  Two detector rows travel as the real and imaginary part of
+// one complex row: the filter's spectrum is real and even, so it acts on both
+// at once.  A thread keeps 16 complex elements in registers; N / 16 threads
+// share a transform of N = R1 R2 R3 points, done in place with decimation in
+// frequency forward and the mirrored decimation in time back, so the spectrum
+// stays in digit-reversed order (the host lays the filter out in that order)
+// and the last forward and the first inverse pass meet in registers: 4 trips
+// through shared memory for 3 radices.  The zero half of the padded row
+// (W <= N / 2) is never loaded, and only the first half is transformed back.
+// Rows move through memory once: 8 bytes per pixel.  384^2 x 512 views, cone,
+// Hamming: 2.47 -> 0.70 ms (0.87 TB/s: the passes'
+// arithmetic and exchanges, not the memory, bound it); 3 CTAs of 80 registers per SM.
+//
+// The filter all but removes a smooth row, so a transform's rounding (relative
+// to the row) would stand out against the output: 2.2e-6 of it at 384 columns,
+// Hamming, against 1.8e-6 for the direct sum.  So the row's differences x[u] -
+// x[u-1] are transformed and the spectrum is divided by 1 - exp(-i w): what is
+// transformed is as small as the output.  The sum of a row, which differences
+// lose, is taken beside them and is the transform's element 0.
+//
+// A row with a value that is not finite or above 1e30 would reach its partner
+// (and could overflow in a sum the direct form does not take): such rows enter
+// the transform as zeros and are convolved directly afterwards.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return tv_sub2(a, b); }
+__device__ __forceinline__ float2 c_mul(float2 a, float2 w) {
+  return make_float2(fmaf(a.x, w.x, -(a.y * w.y)), fmaf(a.x, w.y, a.y * w.x));
+}
+template <bool INV>
+__device__ __forceinline__ float2 c_rot(float2 a) {  // times -i (forward), i (inverse)
+  return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+template <bool INV>
+__device__ __forceinline__ float2 c_conj_if(float2 w) {
+  return INV ? make_float2(w.x, -w.y) : w;
+}
+
+template <bool INV>
+__device__ __forceinline__ void dft4(float2& a, float2& b, float2& c, float2& d) {
+  const float2 t0 = c_add(a, c), t1 = c_sub(a, c), t2 = c_add(b, d), t3 = c_rot<INV>(c_sub(b, d));
+  a = c_add(t0, t2);
+  b = c_add(t1, t3);
+  c = c_sub(t0, t2);
+  d = c_sub(t1, t3);
+}
+
+// R-point transform of v[0 .. R-1], natural order in and out.
+template <int R, bool INV>
+__device__ __forceinline__ void dft(float2* v) {
+  if constexpr (R == 4) {
+    dft4<INV>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 8) {
+    constexpr float h = 0.70710678118654752f;
+    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    dft4<INV>(e[0], e[1], e[2], e[3]);
+    dft4<INV>(o[0], o[1], o[2], o[3]);
+    o[1] = c_mul(o[1], c_conj_if<INV>(make_float2(h, -h)));
+    o[2] = c_rot<INV>(o[2]);
+    o[3] = c_mul(o[3], c_conj_if<INV>(make_float2(-h, -h)));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = c_add(e[k], o[k]);
+      v[k + 4] = c_sub(e[k], o[k]);
+    }
+  } else {
+    static_assert(R == 16, "radix 4, 8 or 16");
+    // cos / sin of pi/8
+    constexpr float c1 = 0.92387953251128676f, s1 = 0.38268343236508977f, h = 0.70710678118654752f;
+    float2 y[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) y[b][a] = v[4 * a + b];
+      dft4<INV>(y[b][0], y[b][1], y[b][2], y[b][3]);
+    }
+    // twiddles exp(-2 pi i b k / 16)
+    y[1][1] = c_mul(y[1][1], c_conj_if<INV>(make_float2(c1, -s1)));
+    y[1][2] = c_mul(y[1][2], c_conj_if<INV>(make_float2(h, -h)));
+    y[1][3] = c_mul(y[1][3], c_conj_if<INV>(make_float2(s1, -c1)));
+    y[2][1] = c_mul(y[2][1], c_conj_if<INV>(make_float2(h, -h)));
+    y[2][2] = c_rot<INV>(y[2][2]);
+    y[2][3] = c_mul(y[2][3], c_conj_if<INV>(make_float2(-h, -h)));
+    y[3][1] = c_mul(y[3][1], c_conj_if<INV>(make_float2(s1, -c1)));
+    y[3][2] = c_mul(y[3][2], c_conj_if<INV>(make_float2(-h, -h)));
+    y[3][3] = c_mul(y[3][3], c_conj_if<INV>(make_float2(-c1, s1)));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      dft4<INV>(y[0][k], y[1][k], y[2][k], y[3][k]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[k + 4 * q] = y[q][k];
+    }
+  }
+}
+
+// v[k] *= exp(-+2 pi i k f / N) for k < R: the powers 1, 2, 4, 8 from the
+// table, the others as products of those (loading every power took 745 us
+// where this takes 625 at 384^2 x 512).
+template <int R, bool INV>
+__device__ __forceinline__ void twiddle(float2* v, const float2* __restrict__ tw, int f) {
+  float2 p[R];
+  p[1] = c_conj_if<INV>(__ldg(tw + f));
+  p[2] = c_conj_if<INV>(__ldg(tw + 2 * f));
+  if constexpr (R > 4) p[4] = c_conj_if<INV>(__ldg(tw + 4 * f));
+  if constexpr (R > 8) p[8] = c_conj_if<INV>(__ldg(tw + 8 * f));
+#pragma unroll
+  for (int k = 1; k < R; ++k) {
+    if (k > 8) p[k] = c_mul(p[8], p[k - 8]);
+    else if (k > 4 && k < 8) p[k] = c_mul(p[4], p[k - 4]);
+    else if (k == 3) p[k] = c_mul(p[2], p[1]);
+    v[k] = c_mul(v[k], p[k]);
+  }
+}
+
+// One spare element per 8 keeps the stride-R passes off each other's banks.
+__device__ __forceinline__ int fft_slot(int i) { return i + (i >> 3); }
+
+// Weighted input sample as prefilter_input, the cosine weight by a reciprocal
+// square root with one Newton step.
+__device__ __forceinline__ float prefilter_fast_input(const FiltArgs& A,
+                                                      const float* __restrict__ sino,
+                                                      const float* __restrict__ pre, size_t gi,
+                                                      int v, int u, float pk) {
+  float s = __ldg(sino + gi);
+  if (A.log_input) {
+    s = -logf(s / __ldg(pre + gi));
+    if (!isfinite(s)) s = 0.f;
+  }
+  if (A.geom != 0) {
+    const float U = (float)(u + 1) - (float)(A.W - 1) * 0.5f;
+    const float V = (float)(v + 1) - (float)(A.H - 1) * 0.5f;
+    const float q = A.geom == 2 ? A.sad * A.sad + U * U + V * V : A.sad * A.sad + U * U;
+    const float r = rsqrtf(q);
+    s *= A.sad * (r * fmaf(-0.5f * q * r, r, 1.5f));
+  }
+  return s * pk;
+}
+
+constexpr int kFftThreads = 256, kFftElems = 16 * kFftThreads;  // complex elements per CTA
+
+template <int R1, int R2, int R3>
+__global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
+    const FiltArgs A, const float* __restrict__ sino, const float* __restrict__ pre,
+    const float* __restrict__ parker, const float* __restrict__ dbeta,
+    const float* __restrict__ kern, float* __restrict__ out, long long pairs) {
+  constexpr int N = R1 * R2 * R3, TF = N / 16, NF = kFftThreads / TF;
+  static_assert(R1 == 16 && kFftThreads % TF == 0, "16 elements per thread");
+  __shared__ float2 sm[kFftElems + kFftElems / 8];
+  __shared__ int bad[2 * NF];  // rows kept out of the transform
+  constexpr int TW = TF < 32 ? TF : 32, NWF = TF / TW;  // lanes and warps per transform
+  __shared__ float2 psum[NF * NWF], edge[8 * NF * NWF];
+  // after the spatial kernel: the differences' spectrum and the twiddles
+  const float2* spec = reinterpret_cast<const float2*>(kern + N);
+  const float2* tw = spec + N;
+  const int n = threadIdx.x % TF, q = threadIdx.x / TF;
+  float2* x = sm + q * (N + N / 8);
+  const int W = A.W, H = A.H, hp = (H + 1) >> 1;
+  const long long pair = (long long)blockIdx.x * NF + q;
+  const bool live = pair < pairs;
+  int view = 0, v0 = 0;
+  if (live) {
+    view = pairs <= 0x7fffffffLL ? (int)((unsigned)pair / (unsigned)hp) : (int)(pair / hp);
+    v0 = 2 * (int)(pair - (long long)view * hp);
+  }
+  const bool two = v0 + 1 < H;
+  const size_t row0 = ((size_t)view * H + v0) * W;
+  if (threadIdx.x < 2 * NF) bad[threadIdx.x] = 0;
+  __syncthreads();
+  float2 e[16];
+  bool b0 = false, b1 = false;
+  {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int u = n + j * TF;
+      float2 s = make_float2(0.f, 0.f);
+      if (live && u < W) {
+        const float pk = __ldg(parker + (size_t)view * W + u);
+        s.x = prefilter_fast_input(A, sino, pre, row0 + u, v0, u, pk);
+        if (two) s.y = prefilter_fast_input(A, sino, pre, row0 + W + u, v0 + 1, u, pk);
+      }
+      b0 |= !(fabsf(s.x) <= 1.0e30f);
+      b1 |= !(fabsf(s.y) <= 1.0e30f);
+      e[j] = s;
+      e[j + 8] = make_float2(0.f, 0.f);
+    }
+    if (b0) bad[2 * q] = 1;
+    if (b1) bad[2 * q + 1] = 1;
+  }
+  // row sums, and each element's left neighbour: lane n - 1, whose warp leaves
+  // its last lane's elements in edge
+  const int wq = q * NWF + n / TW;
+  float2 sum = make_float2(0.f, 0.f), left[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sum = c_add(sum, e[j]);
+#pragma unroll
+  for (int o = TW / 2; o > 0; o >>= 1) {
+    sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+    sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    left[j].x = __shfl_up_sync(0xffffffffu, e[j].x, 1, TW);
+    left[j].y = __shfl_up_sync(0xffffffffu, e[j].y, 1, TW);
+  }
+  if (n % TW == 0) psum[wq] = sum;
+  if (n % TW == TW - 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) edge[8 * wq + j] = e[j];
+  }
+  const bool any = __syncthreads_or(b0 || b1) != 0;
+  const bool bad0 = bad[2 * q] != 0, bad1 = bad[2 * q + 1] != 0;
+  float2 past = make_float2(0.f, 0.f);  // element N / 2 of the differences (thread 0)
+  if (n % TW == 0) {
+    const float2* ed = edge + 8 * (n == 0 ? q * NWF + NWF - 1 : wq - 1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      left[j] = n ? ed[j] : (j ? ed[j - 1] : make_float2(0.f, 0.f));
+    if (n == 0) past = make_float2(-ed[7].x, -ed[7].y);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) e[j] = c_sub(e[j], left[j]);
+  e[8] = past;
+  if (any) {
+#pragma unroll
+    for (int j = 0; j <= 8; ++j) {
+      if (bad0) e[j].x = 0.f;
+      if (bad1) e[j].y = 0.f;
+    }
+  }
+  // radix R1, stride TF
+  dft<R1, false>(e);
+  twiddle<R1, false>(e, tw, n);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) x[fft_slot(n + j * TF)] = e[j];
+  __syncthreads();
+  if constexpr (R3 > 1) {  // radix R2, stride R3
+#pragma unroll
+    for (int i = 0; i < 16 / R2; ++i) {
+      const int b = n + i * TF, t = b % R3, base = (b / R3) * (R2 * R3) + t;
+#pragma unroll
+      for (int j = 0; j < R2; ++j) e[j] = x[fft_slot(base + j * R3)];
+      dft<R2, false>(e);
+      twiddle<R2, false>(e, tw, t * R1);
+#pragma unroll
+      for (int j = 0; j < R2; ++j) x[fft_slot(base + j * R3)] = e[j];
+    }
+    __syncthreads();
+  }
+  {  // last radix, filter, first inverse radix
+    constexpr int RL = R3 > 1 ? R3 : R2;
+#pragma unroll
+    for (int i = 0; i < 16 / RL; ++i) {
+      const int base = (n + i * TF) * RL;
+#pragma unroll
+      for (int j = 0; j < RL; ++j) e[j] = x[fft_slot(base + j)];
+      dft<RL, false>(e);
+      if (base == 0) {  // frequency 0: the row sums (element 0 of the spectrum is real)
+        e[0] = psum[q * NWF];
+#pragma unroll
+        for (int w = 1; w < NWF; ++w) e[0] = c_add(e[0], psum[q * NWF + w]);
+        if (bad0) e[0].x = 0.f;
+        if (bad1) e[0].y = 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < RL; ++j) e[j] = c_mul(e[j], __ldg(spec + base + j));
+      dft<RL, true>(e);
+#pragma unroll
+      for (int j = 0; j < RL; ++j) x[fft_slot(base + j)] = e[j];
+    }
+    __syncthreads();
+  }
+  if constexpr (R3 > 1) {
+#pragma unroll
+    for (int i = 0; i < 16 / R2; ++i) {
+      const int b = n + i * TF, t = b % R3, base = (b / R3) * (R2 * R3) + t;
+#pragma unroll
+      for (int j = 0; j < R2; ++j) e[j] = x[fft_slot(base + j * R3)];
+      twiddle<R2, true>(e, tw, t * R1);
+      dft<R2, true>(e);
+#pragma unroll
+      for (int j = 0; j < R2; ++j) x[fft_slot(base + j * R3)] = e[j];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) e[j] = x[fft_slot(n + j * TF)];
+  twiddle<R1, true>(e, tw, n);
+  dft<R1, true>(e);
+  const float db = live ? __ldg(dbeta + view) : 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int u = n + j * TF;
+    if (live && u < W) {
+      if (!bad0) out[row0 + u] = e[j].x * db;
+      if (two && !bad1) out[row0 + W + u] = e[j].y * db;
+    }
+  }
+  if (any) {  // rows kept out: the direct sum, from staged inputs (out may be sino)
+    __syncthreads();
+    for (int u = n; live && u < W; u += TF)
+      x[u] = make_float2(bad0 ? prefilter_input(A, sino, pre, parker, view, v0, u) : 0.f,
+                         bad1 ? prefilter_input(A, sino, pre, parker, view, v0 + 1, u) : 0.f);
+    __syncthreads();
+    for (int u = n; live && (bad0 || bad1) && u < W; u += TF) {
+      float2 acc = make_float2(0.f, 0.f);
+      for (int j = 0; j < W; ++j) {
+        const float k = __ldg(kern + ((u - j) & (N - 1)));
+        acc = make_float2(fmaf(x[j].x, k, acc.x), fmaf(x[j].y, k, acc.y));
+      }
+      if (bad0) out[row0 + u] = acc.x * db;
+      if (bad1) out[row0 + W + u] = acc.y * db;
+    }
+  }
+}
+
+template <int R1, int R2, int R3>
+static cudaError_t prefilter_fft_go(const FiltArgs& a, const float* sino, const float* pre,
+                                    const float* parker, const float* dbeta, const float* kern,
+                                    float* out, cudaStream_t st) {
+  constexpr int NF = kFftElems / (R1 * R2 * R3);
+  const long long pairs = (long long)a.nP * ((a.H + 1) / 2), ctas = (pairs + NF - 1) / NF;
+  if (ctas > 0x7fffffffLL) return cudaErrorInvalidValue;
+  prefilter_fft_kernel<R1, R2, R3><<<(unsigned)ctas, kFftThreads, 0, st>>>(
+      a, sino, pre, parker, dbeta, kern, out, pairs);
+  return cudaGetLastError();
+}
+
+// Radices of the transform of `order` points: r[0] * r[1] * r[2]; false where
+// the direct form serves (W > 2048).
+bool prefilter_fft_radices(int order, int r[3]) {
+  static const int tab[7][3] = {{16, 4, 1},  {16, 8, 1},  {16, 16, 1}, {16, 8, 4},
+                                {16, 8, 8},  {16, 16, 8}, {16, 16, 16}};
+  for (const auto& t : tab)
+    if (t[0] * t[1] * t[2] == order) {
+      for (int i = 0; i < 3; ++i) r[i] = t[i];
+      return true;
+    }
+  return false;
+}
+
 template <int RG>
 static cudaError_t prefilter_tiled_go(const FiltArgs& a, size_t smem, const float* sino,
                                       const float* pre, const float* parker, const float* dbeta,
@@ -778,15 +1122,29 @@ static cudaError_t prefilter_tiled_go(const FiltArgs& a, size_t smem, const floa
 
 cudaError_t launch_prefilter(const FiltArgs& a, const float* sino,
                              const float* pre, const float* parker,
-                             const float* dbeta, const float* kern, float* out,
+                             const float* dbeta, const float* kern, bool fft, float* out,
                              cudaStream_t st) {
-  // register-blocked form with the most rows per block whose rows and kernel
-  // fit 200 KB of shared memory
+  if (fft) {
+#define FFT(R1, R2, R3)          \
+  if (a.order == R1 * R2 * R3)   \
+  return prefilter_fft_go<R1, R2, R3>(a, sino, pre, parker, dbeta, kern, out, st)
+    FFT(16, 4, 1);
+    FFT(16, 8, 1);
+    FFT(16, 16, 1);
+    FFT(16, 8, 4);
+    FFT(16, 8, 8);
+    FFT(16, 16, 8);
+    FFT(16, 16, 16);
+#undef FFT
+    return cudaErrorInvalidValue;
+  }
+  // rows too long for the transform (W > 2048): the register-blocked direct
+  // form with the most rows per block whose rows and kernel fit 200 KB of
+  // shared memory
   const size_t Wj = (size_t)((a.W + 7) & ~7);
-  for (int rg : {4, 2, 1}) {
+  for (int rg : {2, 1}) {
     const size_t smem = sizeof(float) * ((size_t)a.order + (size_t)8 * rg * Wj);
     if (smem > 200 * 1024) continue;
-    if (rg == 4) return prefilter_tiled_go<4>(a, smem, sino, pre, parker, dbeta, kern, out, st);
     if (rg == 2) return prefilter_tiled_go<2>(a, smem, sino, pre, parker, dbeta, kern, out, st);
     return prefilter_tiled_go<1>(a, smem, sino, pre, parker, dbeta, kern, out, st);
   }

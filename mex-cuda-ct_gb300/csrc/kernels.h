@@ -299,9 +299,13 @@ struct FiltArgs {
   int W, H, nP, order, geom, log_input;
   float sad;
 };
+// kern: the spatial kernel (order floats).  fft: it is followed by the tables
+// of the FFT form (prefilter_fft_radices; 5 order floats in all: see
+// filter_kernel), else the direct convolution runs.
 cudaError_t launch_prefilter(const FiltArgs& a, const float* sino,
                              const float* pre, const float* parker,
-                             const float* dbeta, const float* kern,
+                             const float* dbeta, const float* kern, bool fft,
                              float* out, cudaStream_t st);
+bool prefilter_fft_radices(int order, int r[3]);
 
 }  // namespace mexct

@@ -712,6 +712,12 @@ int filter_order(int W) {
   return order;
 }
 
+// out: the spatial kernel (order floats); where the FFT form serves the order
+// R1 R2 R3, followed by two complex tables of `order` elements: the spectrum
+// of the filter on a row's differences, H / (order (1 - exp(-i w))) (element 0:
+// H[0] / order, for the row's sum), in digit-reversed order (position
+// (k1 R2 + k2) R3 + k3 holds frequency k1 + R1 k2 + R1 R2 k3), and the
+// twiddles exp(-2 pi i k / order).
 void filter_kernel(int W, int filter, double d, std::vector<float>& out) {
   const double pi = 3.14159265358979323846;
   const int order = filter_order(W), half = order / 2;
@@ -749,6 +755,24 @@ void filter_kernel(int W, int filter, double d, std::vector<float>& out) {
     double acc = 0.0;
     for (int m = 0; m < order; ++m) acc += H[m] * ct[((long long)m * n) % order];
     out[n] = (float)(acc / order);
+  }
+  int r[3];
+  if (!prefilter_fft_radices(order, r)) return;
+  out.resize((size_t)5 * order);
+  float* spec = out.data() + order;
+  float* tw = spec + 2 * (size_t)order;
+  for (int k1 = 0; k1 < r[0]; ++k1)
+    for (int k2 = 0; k2 < r[1]; ++k2)
+      for (int k3 = 0; k3 < r[2]; ++k3) {
+        const int f = k1 + r[0] * k2 + r[0] * r[1] * k3;
+        float* s = spec + 2 * (size_t)((k1 * r[1] + k2) * r[2] + k3);
+        // 1 / (1 - exp(-i w)) = (1 - i cot(w / 2)) / 2
+        s[0] = (float)(f ? H[f] / (2.0 * order) : H[0] / order);
+        s[1] = (float)(f ? -H[f] / (2.0 * order * std::tan(pi * f / order)) : 0.0);
+      }
+  for (int k = 0; k < order; ++k) {
+    tw[2 * k] = (float)ct[k];
+    tw[2 * k + 1] = (float)-std::sin(2.0 * pi * k / order);
   }
 }
 
@@ -838,9 +862,12 @@ mexct_status prefilter_dev_impl(mexct_ctx* c, const float* d_sino,
   fa.geom = geom;
   fa.log_input = d_pre ? 1 : 0;
   fa.sad = sad;
+  // tables: kernel (and the FFT form's), Parker window, dbeta / 2
   const float* dt = c->tabs.as<float>();
-  MEXCT_TRY_CUDA(launch_prefilter(fa, d_sino, d_pre, dt + order, dt + order + (size_t)nP * W, dt,
-                                  d_out, st),
+  int radix[3];
+  const bool fft = prefilter_fft_radices(order, radix);
+  const float* dp = dt + (size_t)order * (fft ? 5 : 1);
+  MEXCT_TRY_CUDA(launch_prefilter(fa, d_sino, d_pre, dp, dp + (size_t)nP * W, dt, fft, d_out, st),
                  "prefilter: launch");
   return MEXCT_OK;
 }
@@ -859,9 +886,10 @@ mexct_status prefilter_tables(mexct_ctx* c, int W, int H, int nP, const float* a
   }
   // Parker window per (view, row element) and dbeta/2 per view.
   (void)pi;
-  std::vector<float> tab((size_t)order + (size_t)nP * W + nP);
-  std::memcpy(tab.data(), c->filt_kern.data(), sizeof(float) * order);
-  float* parker = tab.data() + order;
+  const size_t nk = c->filt_kern.size();  // kernel, or kernel + spectrum + twiddles
+  std::vector<float> tab(nk + (size_t)nP * W + nP);
+  std::memcpy(tab.data(), c->filt_kern.data(), sizeof(float) * nk);
+  float* parker = tab.data() + nk;
   float* dbeta = parker + (size_t)nP * W;
   parker_table(W, nP, angles, geom, sad, q, parker);
   for (int i = 0; i < nP; ++i)
