@@ -178,6 +178,7 @@ void fill_std_rays(RayArgs& a, int W, int H, float sad, int geom,
   // 328); voxel/2 for every geometry inside OSC (CUDAmex_oscIter.cu:244).
   a.step = (geom == 2 && !osc) ? 1.0f : 0.5f;
   a.P = (long long)W * H;
+  a.zrows = H + 2;
   a.vstride = 1;
   a.du = 1.0f;                      // the reference's detector: unit pitch,
   a.dv = 1.0f;                      // rays through the pixel centres

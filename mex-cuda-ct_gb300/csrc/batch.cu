@@ -28,6 +28,9 @@ struct mexct_batch {
   std::vector<mexct_problem> probs;
   // BP launch arguments per problem and view chunk (at most kMaxViews views)
   std::vector<std::vector<std::unique_ptr<VoxArgs>>> vox;
+  // parallel / fan FP: launch arguments per problem and view chunk, tensor maps
+  std::vector<std::vector<std::unique_ptr<RayArgs>>> rays;
+  std::vector<CUtensorMap> rmx, rmy;
   Buf fp_desc, trig, counters, err;
   long long fp_items = 0, pad_items = 0;
   int sms = 1;  // set from cudaDevAttrMultiProcessorCount at creation
@@ -78,6 +81,9 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
   b->pads.resize(2 * n);
   b->spads.resize(n);
   b->vox.resize(n);
+  b->rays.resize(n);
+  b->rmx.resize(n);
+  b->rmy.resize(n);
   for (int k = 0; k < mexct_batch::kAux; ++k) {
     MEXCT_TRY_CUDA(cudaStreamCreateWithFlags(&b->aux[k], cudaStreamNonBlocking),
                    "batch_create: streams");
@@ -93,17 +99,35 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
   for (int i = 0; i < n; ++i) {
     const mexct_problem& p = probs[i];
     const int W = p.W, H = p.H;
-    const int Pf = slab_pitch(W);
-    const size_t pb = (size_t)Pf * (W + 2) * (H + 2) * sizeof(float);
-    MEXCT_TRY_CUDA(b->pads[2 * i].ensure(pb), "batch_create: padded volume");
-    MEXCT_TRY_CUDA(b->pads[2 * i + 1].ensure(pb), "batch_create: padded volume");
+    const bool rows = fp_uses_rows(p.geom);
+    const FpLayout L = fp_layout(rows, W, H, kF32);
+    const int Pf = L.pitch;
+    MEXCT_TRY_CUDA(b->pads[2 * i].ensure(L.px), "batch_create: padded volume");
+    MEXCT_TRY_CUDA(b->pads[2 * i + 1].ensure(L.py), "batch_create: padded volume");
     for (int v = 0; v < p.nP; ++v) trig_of(p.angles[v], &trig[toff + v]);
     BatchFp& f = fd[i];
     std::memset(&f, 0, sizeof f);
-    MEXCT_TRY_CUDA(make_slab_tmap(&f.tmx, b->pads[2 * i].p, kF32, Pf, W + 2, H + 2, p.geom),
+    MEXCT_TRY_CUDA(make_fp_tmaps(rows, p.geom, b->pads[2 * i].p, b->pads[2 * i + 1].p, kF32, W, H,
+                                 &f.tmx, &f.tmy),
                    "batch_create: tensor map");
-    MEXCT_TRY_CUDA(make_slab_tmap(&f.tmy, b->pads[2 * i + 1].p, kF32, Pf, W + 2, H + 2, p.geom),
-                   "batch_create: tensor map");
+    if (rows) {
+      b->rmx[i] = f.tmx;
+      b->rmy[i] = f.tmy;
+      const SlabEpi none{nullptr, nullptr, nullptr, nullptr, nullptr};
+      for (int v0 = 0; v0 < p.nP; v0 += kMaxViews) {
+        std::unique_ptr<RayArgs> ra(new RayArgs);
+        fill_std_rays(*ra, W, H, p.sad, p.geom, false);
+        if (v0 == 0)  // kernel attributes, before any capture
+          MEXCT_TRY_CUDA(launch_fp_rows(p.geom, 0, *ra, f.tmx, f.tmy, b->pads[2 * i].p, Pf, kF32,
+                                        nullptr, kF32, none, nullptr),
+                         "batch_create: kernel setup");
+        ra->nall = p.nP;
+        ra->nviews = std::min(kMaxViews, p.nP - v0);
+        ra->view0 = v0;
+        for (int v = 0; v < ra->nviews; ++v) trig_of(p.angles[v0 + v], &ra->trig[v]);
+        b->rays[i].push_back(std::move(ra));
+      }
+    }
     f.W = W;
     f.H = H;
     f.geom = p.geom;
@@ -118,7 +142,8 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
     f.sad = p.sad;
     f.step = p.geom == 2 ? 1.0f : 0.5f;
     f.item0 = b->fp_items;
-    b->fp_items += (long long)p.nP * f.tiles_u * ((H + 7) / 8);
+    // parallel / fan problems have launches of their own: no items here
+    if (!rows) b->fp_items += (long long)p.nP * f.tiles_u * ((H + 7) / 8);
     f.px = b->pads[2 * i].p;
     f.py = b->pads[2 * i + 1].p;
     f.out = p.d_sino;
@@ -126,7 +151,7 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
     f.vol = p.d_vol;
     f.pad_item0 = b->pad_items;
     const long long nt = (Pf + 31) / 32;
-    b->pad_items += nt * nt * (H + 2);
+    if (!rows) b->pad_items += nt * nt * (H + 2);
     // BP: views in the quad layout, one launch per kMaxViews views
     // (mexct_bp_dev's shapes without view blocks)
     MEXCT_TRY_CUDA(b->spads[i].ensure(sino_pad_elems(W, H, p.nP) * sizeof(float4)),
@@ -158,6 +183,25 @@ mexct_status mexct_batch_fp(mexct_batch* b, void* stream) {
   DevGuard dg(b->device);
   NvtxRange nvtx("mexct:batch_fp");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // parallel / fan problems beside the persistent launch of the cone problems,
+  // on the streams the BP uses
+  MEXCT_TRY_CUDA(cudaEventRecord(b->fork, st), "batch_fp: fork");
+  bool used[mexct_batch::kAux] = {};
+  for (int i = 0, k = 0; i < b->n; ++i) {
+    if (b->rays[i].empty()) continue;
+    const mexct_problem& p = b->probs[i];
+    const int q = k++ % mexct_batch::kAux;
+    cudaStream_t s = b->aux[q];
+    if (!used[q]) MEXCT_TRY_CUDA(cudaStreamWaitEvent(s, b->fork, 0), "batch_fp: fork");
+    used[q] = true;
+    MEXCT_TRY_CUDA(launch_pad_rows(p.d_vol, kF32, p.W, p.H, false, b->pads[2 * i].p, s),
+                   "batch_fp: padding");
+    SlabEpi e{nullptr, nullptr, nullptr, nullptr, b->err.as<unsigned>()};
+    for (const auto& ra : b->rays[i])
+      MEXCT_TRY_CUDA(launch_fp_rows(p.geom, 0, *ra, b->rmx[i], b->rmy[i], b->pads[2 * i].p,
+                                    rows_pitch(p.H, kF32), kF32, p.d_sino, kF32, e, s),
+                     "batch_fp: launch");
+  }
   MEXCT_TRY_CUDA(launch_pad_batch(b->fp_desc.as<BatchFp>(), b->n, b->pad_items, st),
                  "batch_fp: padding");
   MEXCT_TRY_CUDA(cudaMemsetAsync(b->counters.p, 0, sizeof(unsigned long long), st),
@@ -166,6 +210,11 @@ mexct_status mexct_batch_fp(mexct_batch* b, void* stream) {
                                  b->counters.as<unsigned long long>(), b->err.as<unsigned>(),
                                  b->sms * slab_ctas_per_sm(), st),
                  "batch_fp: launch");
+  for (int k = 0; k < mexct_batch::kAux; ++k) {
+    if (!used[k]) continue;
+    MEXCT_TRY_CUDA(cudaEventRecord(b->join[k], b->aux[k]), "batch_fp: join");
+    MEXCT_TRY_CUDA(cudaStreamWaitEvent(st, b->join[k], 0), "batch_fp: join");
+  }
   return MEXCT_OK;
 }
 

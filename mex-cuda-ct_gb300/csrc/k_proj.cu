@@ -997,7 +997,10 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
       const float f = ldp(o);
       const float m = fmaxf(f + (f * num[j] / den[j]), 0.f);
       stf(o, m);
-      if (padx) {
+      if (GEOM < 2 && !DET) {
+        // the parallel / fan FP's z-fastest layout (columns of pitch Pf)
+        if (padx) stf(padx + ((size_t)(iy + 1) * Ps + (ix + 1)) * Pf + z, m);
+      } else if (padx) {
         // the slab FP's padded layouts: x-fastest and y-fastest, frame of one
         const size_t zp = (size_t)(z + 1) * Ps;
         stf(padx + (size_t)(ix + 1) + (size_t)Pf * ((size_t)(iy + 1) + zp), m);

@@ -41,6 +41,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "tma.cuh"
 
 namespace mexct {
 
@@ -159,111 +160,18 @@ cudaError_t launch_pad_volume(const void* src, int dtype, int W, int H, int Pf,
   return cudaGetLastError();
 }
 
-cudaError_t launch_pad_volume_sub(const float* src, int W, int nz, int Pf, bool zero_lo,
+cudaError_t launch_pad_volume_sub(bool rows, const float* src, int W, int nz, bool zero_lo,
                                   bool zero_hi, float* px, float* py, cudaStream_t st,
                                   bool border) {
-  const int Ps = W + 2, Pz = nz + 2;
+  if (rows)
+    return launch_pad_rows(src, kF32, W, nz, border, px, st);
+  const int Ps = W + 2, Pz = nz + 2, Pf = slab_pitch(W);
   dim3 blk(32, 8), g1((Pf + 31) / 32, (Ps + 7) / 8, Pz);
   dim3 g2((Pf + 31) / 32, (Pf + 31) / 32, Pz);
   const int mode = border ? 1 : ((zero_lo ? 2 : 0) | (zero_hi ? 4 : 0));
   pad_x_kernel<float><<<g1, blk, 0, st>>>(src, px, W, nz, Pf, mode);
   pad_transpose_kernel<float><<<g2, blk, 0, st>>>(px, py, Ps, Pf);
   return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// TMA / mbarrier helpers (inline PTX).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1,
-                                            int c2, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Non-blocking test of a phase (try_wait may suspend the thread for a while).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// After a CTA gave up waiting: copies issued before still land in its
-// buffers, so wait (at most 2 s each) until the last copy issued into each
-// buffer has completed.  Copies into one buffer complete in order, so the
-// last one's phase parity is (count - 1) & 1.  issued: 16-bit counts per
-// buffer.  Kept out of line: it only runs after a failure.
-__device__ __noinline__ void slab_drain(uint64_t* bar, uint32_t issued, unsigned* err) {
-  for (int b = 0; b < 2; ++b) {
-    const uint32_t n = (issued >> (16 * b)) & 0xffffu;
-    if (n == 0) continue;
-    const uint64_t t0 = global_ns();
-    bool done = false;
-    do {
-      done = mbar_try_wait(&bar[b], (n - 1u) & 1u);
-    } while (!done && global_ns() - t0 < 2000000000ull);
-    if (!done && err) atomicOr(err, 2u);
-  }
-}
-
-// Bounded wait: after one attempt, keeps trying for at most wait_us
-// microseconds of wall time (default 2 s; < 0: one non-blocking test only), then records the
-// failure in err and in the CTA's abort flag and reports it to the caller,
-// which samples the slab from global memory instead (the result is the same).
-// Once a CTA has given up, its later waits return at once and no further
-// copies are issued, so a broken pipeline costs one time-out per CTA.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, unsigned* err,
-                                                  volatile int* abort, int wait_us) {
-  if (*abort) return false;
-  if (wait_us < 0) {
-    if (mbar_test_wait(bar, parity)) return true;
-  } else {
-    // the usual short waits end here, without reading the clock
-    for (int i = 0; i < 64; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t limit = wait_us > 0 ? (uint64_t)wait_us * 1000ull : 2000000000ull;
-    const uint64_t t0 = global_ns();
-    while (global_ns() - t0 < limit)
-      if (mbar_try_wait(bar, parity)) return true;
-  }
-  *abort = 1;
-  if (err) atomicOr(err, 1u);
-  return false;
 }
 
 // ---------------------------------------------------------------------------
@@ -1159,9 +1067,7 @@ __global__ void __launch_bounds__(256, kSlabCtas) fp_batch_kernel(
     J.tu0 = (tile % B.tiles_u) * 32;
     J.tv0 = (tile / B.tiles_u) * 8;
     J.tmx = &B.tmx; J.tmy = &B.tmy; J.px = B.px; J.py = B.py; J.out = B.out;
-    if (B.geom == 0) slab_tile<0, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
-    else if (B.geom == 1) slab_tile<1, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
-    else slab_tile<2, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
+    slab_tile<2, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
   }
 }
 
@@ -1203,6 +1109,24 @@ cudaError_t make_slab_tmap(CUtensorMap* map, const void* base, int dtype, int Pf
 }
 
 int slab_pitch(int W) { return ((W + 2 + 7) / 8) * 8; }
+
+FpLayout fp_layout(bool rows, int W, int nz, int dtype) {
+  if (rows) return {rows_bytes(W, nz, dtype), 0, rows_pitch(nz, dtype)};
+  const int Pf = slab_pitch(W);
+  const size_t b = (size_t)Pf * (W + 2) * (nz + 2) * (dtype == kF32 ? 4 : 2);
+  return {b, b, Pf};
+}
+
+cudaError_t make_fp_tmaps(bool rows, int geom, const void* px, const void* py, int dtype, int W,
+                          int nz, CUtensorMap* mx, CUtensorMap* my) {
+  if (rows) {
+    cudaError_t e = make_rows_tmap(mx, px, dtype, W, nz, true);
+    return e != cudaSuccess ? e : make_rows_tmap(my, px, dtype, W, nz, false);
+  }
+  const int Pf = slab_pitch(W);
+  cudaError_t e = make_slab_tmap(mx, px, dtype, Pf, W + 2, nz + 2, geom);
+  return e != cudaSuccess ? e : make_slab_tmap(my, py, dtype, Pf, W + 2, nz + 2, geom);
+}
 
 // Whether views 2i and 2i+1 of a launch share their slab boxes: the box
 // covers a tile's bundle with ~18 voxels to spare along f, and two views
@@ -1309,10 +1233,19 @@ cudaError_t launch_fp_slab_g3d(const RayArgs& a, const CUtensorMap& mx, const CU
 cudaError_t launch_fp_slab_sub(int geom, const RayArgs& a, const CUtensorMap& mx,
                                const CUtensorMap& my, const void* px, const void* py, int Pf,
                                float* out, const SlabEpi& e, cudaStream_t st) {
-  if (geom == 0)
-    return slab_go<0, false, 0, float, float, false, true>(a, mx, my, px, py, Pf, out, e, st);
-  if (geom == 1)
-    return slab_go<1, false, 0, float, float, false, true>(a, mx, my, px, py, Pf, out, e, st);
+  if (fp_uses_rows(geom)) {
+    // a slab's rays reach its own rows only: the others' integrals are zero
+    const int lo = a.zoff, hi = a.zoff + a.zrows - 2;  // rows lo .. hi - 1
+    for (int part = 0; part < 2 && !a.accum && a.nviews > 0; ++part) {
+      const size_t row = part ? hi : 0, rows = part ? a.det_h - hi : lo;
+      if (rows == 0) continue;
+      cudaError_t r = cudaMemset2DAsync(
+          out + (size_t)a.view0 * a.P + row * a.det_w, (size_t)a.P * a.vstride * sizeof(float), 0,
+          rows * a.det_w * sizeof(float), a.nviews, st);
+      if (r != cudaSuccess) return r;
+    }
+    return launch_fp_rows(geom, 0, a, mx, my, px, Pf, kF32, out, kF32, e, st);
+  }
   if (geom == 2)
     return slab_go<2, false, 0, float, float, false, true>(a, mx, my, px, py, Pf, out, e, st);
   return cudaErrorInvalidValue;
@@ -1322,20 +1255,12 @@ cudaError_t launch_fp_slab_objective(int geom, const RayArgs& a, const CUtensorM
                                      const CUtensorMap& my, const void* px, const void* py,
                                      int Pf, int vt, const SlabEpi& e, cudaStream_t st) {
   if (!e.obj || !e.pre || !e.post) return cudaErrorInvalidValue;
-#define GO(G, TV) return slab_go<G, true, 2, TV, float>(a, mx, my, px, py, Pf, nullptr, e, st)
-  if (vt == kF32) {
-    if (geom == 0) GO(0, float);
-    if (geom == 1) GO(1, float);
-    GO(2, float);
-  }
-  if (vt == kF16) {
-    if (geom == 0) GO(0, __half);
-    if (geom == 1) GO(1, __half);
-    GO(2, __half);
-  }
-  if (geom == 0) GO(0, __nv_bfloat16);
-  if (geom == 1) GO(1, __nv_bfloat16);
-  GO(2, __nv_bfloat16);
+  if (fp_uses_rows(geom))
+    return launch_fp_rows(geom, 2, a, mx, my, px, Pf, vt, nullptr, kF32, e, st);
+#define GO(TV) return slab_go<2, true, 2, TV, float>(a, mx, my, px, py, Pf, nullptr, e, st)
+  if (vt == kF32) GO(float);
+  if (vt == kF16) GO(__half);
+  GO(__nv_bfloat16);
 #undef GO
 }
 
@@ -1343,55 +1268,25 @@ cudaError_t launch_fp_slab(int geom, bool border, bool osc, const RayArgs& a,
                            const CUtensorMap& mx, const CUtensorMap& my, const void* px,
                            const void* py, int Pf, int vt, void* out, int ot,
                            const SlabEpi& e, cudaStream_t st) {
-#define GO(G, B, EP, TV, TO) return slab_go<G, B, EP, TV, TO>(a, mx, my, px, py, Pf, out, e, st)
+  (void)border;
+  if (fp_uses_rows(geom))
+    return launch_fp_rows(geom, osc ? 1 : 0, a, mx, my, px, Pf, vt, out, ot, e, st);
+#define GO(B, EP, TV, TO) return slab_go<2, B, EP, TV, TO>(a, mx, my, px, py, Pf, out, e, st)
   if (osc) {
     // ot: storage of the residual views (FP16 with FP32 mu only)
     if (ot == kF16) {
       if (vt != kF32) return cudaErrorInvalidValue;
-      if (geom == 0) GO(0, true, 1, float, __half);
-      if (geom == 1) GO(1, true, 1, float, __half);
-      GO(2, true, 1, float, __half);
+      GO(true, 1, float, __half);
     }
-    if (vt == kF32) {
-      if (geom == 0) GO(0, true, 1, float, float);
-      if (geom == 1) GO(1, true, 1, float, float);
-      GO(2, true, 1, float, float);
-    }
-    if (vt == kF16) {
-      if (geom == 0) GO(0, true, 1, __half, float);
-      if (geom == 1) GO(1, true, 1, __half, float);
-      GO(2, true, 1, __half, float);
-    }
-    if (geom == 0) GO(0, true, 1, __nv_bfloat16, float);
-    if (geom == 1) GO(1, true, 1, __nv_bfloat16, float);
-    GO(2, true, 1, __nv_bfloat16, float);
+    if (vt == kF32) GO(true, 1, float, float);
+    if (vt == kF16) GO(true, 1, __half, float);
+    GO(true, 1, __nv_bfloat16, float);
   }
-  (void)border;
-  if (vt == kF32 && ot == kF32) {
-    if (geom == 0) GO(0, false, 0, float, float);
-    if (geom == 1) GO(1, false, 0, float, float);
-    GO(2, false, 0, float, float);
-  }
-  if (vt == kF16 && ot == kF16) {
-    if (geom == 0) GO(0, false, 0, __half, __half);
-    if (geom == 1) GO(1, false, 0, __half, __half);
-    GO(2, false, 0, __half, __half);
-  }
-  if (vt == kF16 && ot == kF32) {
-    if (geom == 0) GO(0, false, 0, __half, float);
-    if (geom == 1) GO(1, false, 0, __half, float);
-    GO(2, false, 0, __half, float);
-  }
-  if (vt == kBF16 && ot == kBF16) {
-    if (geom == 0) GO(0, false, 0, __nv_bfloat16, __nv_bfloat16);
-    if (geom == 1) GO(1, false, 0, __nv_bfloat16, __nv_bfloat16);
-    GO(2, false, 0, __nv_bfloat16, __nv_bfloat16);
-  }
-  if (vt == kBF16 && ot == kF32) {
-    if (geom == 0) GO(0, false, 0, __nv_bfloat16, float);
-    if (geom == 1) GO(1, false, 0, __nv_bfloat16, float);
-    GO(2, false, 0, __nv_bfloat16, float);
-  }
+  if (vt == kF32 && ot == kF32) GO(false, 0, float, float);
+  if (vt == kF16 && ot == kF16) GO(false, 0, __half, __half);
+  if (vt == kF16 && ot == kF32) GO(false, 0, __half, float);
+  if (vt == kBF16 && ot == kBF16) GO(false, 0, __nv_bfloat16, __nv_bfloat16);
+  if (vt == kBF16 && ot == kF32) GO(false, 0, __nv_bfloat16, float);
 #undef GO
   return cudaErrorInvalidValue;
 }

@@ -17,6 +17,8 @@ struct RayArgs {
   float bx, by, bz;        // volume corner -S/2, -S/2, -Z/2
   float SR, RD, step;
   int nviews;              // views in this launch
+  int nall;                // views of the call (0: this launch's), for rules that
+                           // must not depend on how it is split into launches
   int view0, vstride;      // launch view i is global view view0 + i*vstride
   long long P;             // det_w * det_h
   int pts_per_view;        // general3D: per-view points
@@ -166,9 +168,38 @@ cudaError_t launch_fp_slab_sub(int geom, const RayArgs& a, const CUtensorMap& mx
 // the slab are zero where zero_lo / zero_hi (an inner slab face), else edge
 // copies (the volume's own face, clamp addressing); with border the whole
 // frame is zero (border addressing).
-cudaError_t launch_pad_volume_sub(const float* src, int W, int nz, int Pf, bool zero_lo,
+// rows: the z-fastest layout into px.
+cudaError_t launch_pad_volume_sub(bool rows, const float* src, int W, int nz, bool zero_lo,
                                   bool zero_hi, float* px, float* py, cudaStream_t st,
                                   bool border = false);
+
+// Parallel / fan FP over the z-fastest layout (k_rows.cu) of a.zrows - 2 slices
+// starting at whole-volume slice a.zoff.  epi 0: line integrals into out
+// (a.accum adds), 1: OSC residuals, 2: objective partials (one per CTA, at
+// most a.nviews x the slab kernel's tiles of them).  The detector's rows are
+// the volume's slices.  nviews = 0 sets the kernels' attributes only.
+int rows_pitch(int nz, int dtype);            // elements of a column of nz slices
+size_t rows_bytes(int W, int nz, int dtype);  // the layout of a W x W x nz volume
+// border: zeros in the x / y frame, else edge copies (no frame in z).
+cudaError_t launch_pad_rows(const void* src, int dtype, int W, int nz, bool border, void* dst,
+                            cudaStream_t st);
+cudaError_t make_rows_tmap(CUtensorMap* map, const void* base, int dtype, int W, int nz,
+                           bool xdom);
+cudaError_t launch_fp_rows(int geom, int epi, const RayArgs& a, const CUtensorMap& mx,
+                           const CUtensorMap& my, const void* vol, int Ph, int vt, void* out,
+                           int ot, const SlabEpi& e, cudaStream_t st);
+
+// The volume layouts that the FP of a geometry reads.  Rays that stay in a
+// slice (parallel, fan) read one z-fastest copy (rows: px, and py is unused);
+// cone and general3D rays read the x-fastest and y-fastest copies.
+inline bool fp_uses_rows(int geom) { return geom == 0 || geom == 1; }
+struct FpLayout {
+  size_t px, py;  // bytes
+  int pitch;      // the launches' Pf
+};
+FpLayout fp_layout(bool rows, int W, int nz, int dtype);
+cudaError_t make_fp_tmaps(bool rows, int geom, const void* px, const void* py, int dtype, int W,
+                          int nz, CUtensorMap* mx, CUtensorMap* my);
 
 cudaError_t launch_fp_tex(int geom, const RayArgs& a,
                           cudaTextureObject_t tex, float* out,

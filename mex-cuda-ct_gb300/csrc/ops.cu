@@ -94,28 +94,27 @@ namespace mexct {
 // Padded copies of a W x W x H volume in both layouts (clamp: replicated edge;
 // border: zeros) in the given buffers, and TMA maps over them.
 mexct_status prepare_slab_bufs(Buf& px, Buf& py, Buf& err, const void* d_vol, int vt, int W,
-                               int H, bool border, int geom, CUtensorMap* mx, CUtensorMap* my,
-                               int* Pf_out, cudaStream_t st) {
-  const int Pf = slab_pitch(W);
-  const size_t bytes = (size_t)Pf * (W + 2) * (H + 2) * dsize(vt);
-  MEXCT_TRY_CUDA(px.ensure(bytes), "fp: workspace");
-  MEXCT_TRY_CUDA(py.ensure(bytes), "fp: workspace");
+                               int H, bool border, int geom, bool rows, CUtensorMap* mx,
+                               CUtensorMap* my, int* Pf_out, cudaStream_t st) {
+  const FpLayout L = fp_layout(rows, W, H, vt);
+  MEXCT_TRY_CUDA(px.ensure(L.px), "fp: workspace");
+  MEXCT_TRY_CUDA(py.ensure(L.py), "fp: workspace");
   if (!err.p) {
     MEXCT_TRY_CUDA(err.ensure(64), "fp: workspace");
     MEXCT_TRY_CUDA(cudaMemset(err.p, 0, 64), "fp: workspace");
   }
-  MEXCT_TRY_CUDA(launch_pad_volume(d_vol, vt, W, H, Pf, border, px.p, py.p, st),
+  MEXCT_TRY_CUDA(rows ? launch_pad_rows(d_vol, vt, W, H, border, px.p, st)
+                      : launch_pad_volume(d_vol, vt, W, H, L.pitch, border, px.p, py.p, st),
                  "fp: pad volume");
-  MEXCT_TRY_CUDA(make_slab_tmap(mx, px.p, vt, Pf, W + 2, H + 2, geom), "fp: tensor map");
-  MEXCT_TRY_CUDA(make_slab_tmap(my, py.p, vt, Pf, W + 2, H + 2, geom), "fp: tensor map");
-  *Pf_out = Pf;
+  MEXCT_TRY_CUDA(make_fp_tmaps(rows, geom, px.p, py.p, vt, W, H, mx, my), "fp: tensor map");
+  *Pf_out = L.pitch;
   return MEXCT_OK;
 }
 
 mexct_status prepare_slab(mexct_ctx* c, const void* d_vol, int vt, int W, int H,
-                          bool border, int geom, CUtensorMap* mx, CUtensorMap* my, int* Pf_out,
-                          cudaStream_t st) {
-  return prepare_slab_bufs(c->padx, c->pady, c->err, d_vol, vt, W, H, border, geom, mx, my,
+                          bool border, int geom, bool rows, CUtensorMap* mx, CUtensorMap* my,
+                          int* Pf_out, cudaStream_t st) {
+  return prepare_slab_bufs(c->padx, c->pady, c->err, d_vol, vt, W, H, border, geom, rows, mx, my,
                            Pf_out, st);
 }
 
@@ -151,6 +150,7 @@ mexct_status fp_run(mexct_ctx* c, const void* d_vol, int vt, int W, int H, float
   if (nP == 0) return MEXCT_OK;
   std::unique_ptr<RayArgs> a(new RayArgs);
   fill_std_rays(*a, W, H, sad, geom, false);
+  a->nall = nP;
   if (variant == MEXCT_FP_TEXTURE) {
     if (vt != kF32 || ot != kF32)
       return set_err(MEXCT_ERR_UNSUPPORTED, "fp(texture): FP32 storage only");
@@ -159,7 +159,8 @@ mexct_status fp_run(mexct_ctx* c, const void* d_vol, int vt, int W, int H, float
   if (variant == MEXCT_FP_EXPLICIT) {
     CUtensorMap mx, my;
     int Pf = 0;
-    mexct_status s = prepare_slab(c, d_vol, vt, W, H, false, geom, &mx, &my, &Pf, st);
+    mexct_status s = prepare_slab(c, d_vol, vt, W, H, false, geom, fp_uses_rows(geom), &mx, &my,
+                                  &Pf, st);
     if (s) return s;
     SlabEpi e{nullptr, nullptr, nullptr, nullptr, c->err.as<unsigned>(), c->wait_us};
     // launches of at most kMaxViews views, or hook->chunks launches
@@ -336,6 +337,7 @@ mexct_status fp_det_impl(mexct_ctx* c, const float* d_vol, int W, int H, float s
   if (!c || nP == 0) return MEXCT_OK;
   std::unique_ptr<RayArgs> a(new RayArgs);
   fill_std_rays(*a, W, H, sad, geom, false);
+  a->nall = nP;
   a->det_w = det->det_w;
   a->det_h = det->det_h;
   a->u0 = float(det->det_w - 1) / 2;
@@ -345,9 +347,11 @@ mexct_status fp_det_impl(mexct_ctx* c, const float* d_vol, int W, int H, float s
   a->dv = det->dv;
   CUtensorMap mx, my;
   int Pf = 0;
-  mexct_status s = prepare_slab(c, d_vol, kF32, W, H, false, geom, &mx, &my, &Pf, st);
-  if (s) return s;
   const int ss = det->ss;
+  // rows that are the volume's slices: the z-fastest kernel, as the standard FP
+  const bool rows = fp_uses_rows(geom) && ss == 1 && det->dv == 1.0f && det->det_h == H;
+  mexct_status s = prepare_slab(c, d_vol, kF32, W, H, false, geom, rows, &mx, &my, &Pf, st);
+  if (s) return s;
   const long long M = a->P * nP;
   float* dst = d_out;
   if (ss > 1) {
@@ -364,7 +368,10 @@ mexct_status fp_det_impl(mexct_ctx* c, const float* d_vol, int W, int H, float s
         a->nviews = std::min(kMaxViews, nP - v0);
         a->view0 = v0;
         for (int i = 0; i < a->nviews; ++i) trig_of(angles[v0 + i], &a->trig[i]);
-        MEXCT_TRY_CUDA(launch_fp_slab_det(geom, *a, mx, my, c->padx.p, c->pady.p, Pf, dst, e, st),
+        MEXCT_TRY_CUDA(rows ? launch_fp_rows(geom, 0, *a, mx, my, c->padx.p, Pf, kF32, dst, kF32, e,
+                                             st)
+                            : launch_fp_slab_det(geom, *a, mx, my, c->padx.p, c->pady.p, Pf, dst, e,
+                                                 st),
                        "fp: launch");
       }
       if (ss > 1)
@@ -450,8 +457,8 @@ mexct_status g3d_fp_dev_impl(mexct_ctx* c, const float* d_vol, int S, int Z,
   a->pts = d_pts;
   CUtensorMap mx, my;
   int Pf = 0;
-  mexct_status s = prepare_slab(c, d_vol, kF32, S, Z, /*border=*/true, /*geom=*/3, &mx, &my,
-                                &Pf, st);
+  mexct_status s = prepare_slab(c, d_vol, kF32, S, Z, /*border=*/true, /*geom=*/3,
+                                /*rows=*/false, &mx, &my, &Pf, st);
   if (s) return s;
   SlabEpi e{nullptr, nullptr, nullptr, nullptr, c->err.as<unsigned>(), c->wait_us};
   for (int v0 = 0; v0 < nP; v0 += kMaxViews) {
@@ -520,7 +527,8 @@ mexct_status osc_det_impl(mexct_ctx* c, float* d_mu, const float* d_pre, const f
   MEXCT_TRY_CUDA(cudaMemsetAsync(c->r2.p, 0, rbytes, st), "osc_iter_det: workspace");
   CUtensorMap mx, my;
   int Pf = 0;
-  mexct_status ps = prepare_slab(c, d_mu, kF32, W, H, /*border=*/true, geom, &mx, &my, &Pf, st);
+  mexct_status ps = prepare_slab(c, d_mu, kF32, W, H, /*border=*/true, geom, /*rows=*/false, &mx, &my,
+                                 &Pf, st);
   if (ps) return ps;
   std::unique_ptr<RayArgs> ra(new RayArgs);
   std::unique_ptr<VoxArgs> va(new VoxArgs);
@@ -625,7 +633,8 @@ mexct_status osc_dev_impl(mexct_ctx* c, float* d_mu, int mu_type,
   // copies along with mu.
   CUtensorMap mx, my;
   int Pf = 0;
-  mexct_status ps = prepare_slab(c, d_mu, mu_type, W, H, /*border=*/true, geom, &mx, &my, &Pf, st);
+  mexct_status ps = prepare_slab(c, d_mu, mu_type, W, H, /*border=*/true, geom, fp_uses_rows(geom),
+                                 &mx, &my, &Pf, st);
   if (ps) return ps;
   std::unique_ptr<RayArgs> ra(new RayArgs);
   std::unique_ptr<VoxArgs> va(new VoxArgs);

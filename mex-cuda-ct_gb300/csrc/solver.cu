@@ -125,7 +125,7 @@ mexct_status enqueue_objective(mexct_osctv* s, cudaStream_t st) {
   CUtensorMap mx, my;
   int Pf = 0;
   mexct_status ps = prepare_slab_bufs(s->padx, s->pady, s->err, s->mu.p, s->mu_type, s->W, s->H,
-                                      /*border=*/true, s->geom, &mx, &my, &Pf, st);
+                                      /*border=*/true, s->geom, fp_uses_rows(s->geom), &mx, &my, &Pf, st);
   if (ps) return ps;
   std::unique_ptr<RayArgs> ra(new RayArgs);
   fill_std_rays(*ra, s->W, s->H, s->sad, s->geom, /*osc=*/true);
@@ -168,7 +168,7 @@ mexct_status enqueue_iteration(mexct_osctv* s, bool k_gt1, int nsub,
   CUtensorMap mx, my;
   int Pf = 0;
   mexct_status ps = prepare_slab_bufs(s->padx, s->pady, s->err, s->mu.p, s->mu_type, s->W, s->H,
-                                      /*border=*/true, s->geom, &mx, &my, &Pf, st);
+                                      /*border=*/true, s->geom, fp_uses_rows(s->geom), &mx, &my, &Pf, st);
   if (ps) return ps;
   for (int si = 0; si < nsub; ++si) {
     const int sel = picks[si];
@@ -279,13 +279,13 @@ mexct_status mexct_osctv_create_ex(mexct_ctx* ctx, const float* d_pre, const flo
   // and destroying solvers never synchronises the device (other streams keep
   // running); the caller's stream waits for the allocations.
   cudaStream_t a = s->own;
-  const size_t pb = (size_t)slab_pitch(W) * (W + 2) * (H + 2) * dsize(mu_type);
+  const FpLayout lay = fp_layout(fp_uses_rows(geom), W, H, mu_type);
   const size_t parts = std::max<size_t>(tv_partials_needed(W, W, H), ssd_partials_needed()) + 8;
   MEXCT_TRY_CUDA(s->mu.ensure_async(vb, a), "osctv_create: mu");
   MEXCT_TRY_CUDA(s->mu_old.ensure_async(vb, a), "osctv_create: mu_old");
   MEXCT_TRY_CUDA(s->tvbuf.ensure_async(vb, a), "osctv_create: tv");
-  MEXCT_TRY_CUDA(s->padx.ensure_async(pb, a), "osctv_create: padded mu");
-  MEXCT_TRY_CUDA(s->pady.ensure_async(pb, a), "osctv_create: padded mu");
+  MEXCT_TRY_CUDA(s->padx.ensure_async(lay.px, a), "osctv_create: padded mu");
+  MEXCT_TRY_CUDA(s->pady.ensure_async(lay.py, a), "osctv_create: padded mu");
   MEXCT_TRY_CUDA(s->pre.ensure_async(M * 4, a), "osctv_create: pre");
   MEXCT_TRY_CUDA(s->post.ensure_async(M * 4, a), "osctv_create: post");
   // the residual views are sized by mexct_osctv_run for its largest subset
@@ -334,7 +334,7 @@ mexct_status mexct_osctv_create_ex(mexct_ctx* ctx, const float* d_pre, const flo
     CUtensorMap mx, my;
     int Pf = 0;
     mexct_status ps = prepare_slab_bufs(s->padx, s->pady, s->err, s->mu.p, mu_type, W, H, true,
-                                        geom, &mx, &my, &Pf, st);
+                                        geom, fp_uses_rows(geom), &mx, &my, &Pf, st);
     if (ps) return ps;
     std::unique_ptr<RayArgs> ra(new RayArgs);
     fill_std_rays(*ra, W, H, sad, geom, true);

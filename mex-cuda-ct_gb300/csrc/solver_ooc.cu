@@ -61,7 +61,8 @@ SetLayout set_layout(int W, int nz) {
   SetLayout L;
   L.x = al((size_t)(nz + 2) * plane);  // the slab, one halo slice each side (TV)
   const size_t y = al((size_t)(nz + 3) * plane);  // x_{t+1}: two carried slices + slab + halo
-  const size_t pad = 2 * al((size_t)slab_pitch(W) * (W + 2) * (nz + 2) * 4);  // FP layouts
+  // FP layouts (the larger of the geometries')
+  const size_t pad = std::max(2 * al(fp_layout(false, W, nz, kF32).px), al(rows_bytes(W, nz, kF32)));
   L.work = std::max(y, pad);
   L.old = al((size_t)nz * plane);  // mu_old of the slab (||mu_old - mu||)
   L.total = L.x + L.work + L.old;
@@ -248,8 +249,8 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
   }
   if ((size_t)(q - static_cast<unsigned char*>(db.p)) > total)
     return set_err(MEXCT_ERR_CUDA, "osc_tv_ooc: internal layout error");
-  const int Pf = slab_pitch(W);
-  const size_t pad_half = al((size_t)Pf * (W + 2) * (nz + 2) * 4) / 4;  // floats
+  const bool rows = fp_uses_rows(geom);  // one z-fastest layout, else two
+  const size_t pad_half = rows ? 0 : al(fp_layout(false, W, nz, kF32).px) / 4;  // floats
 
   Streams S;
   MEXCT_TRY_CUDA(cudaStreamCreateWithFlags(&S.st, cudaStreamNonBlocking), "osc_tv_ooc: stream");
@@ -316,14 +317,16 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
     ra->zlo = (float)z0;
     ra->zhi = (float)(z0 + m + 1);
     ra->accum = accum ? 1 : 0;
+    ra->nall = nv;
     CUtensorMap mx, my;
-    MEXCT_TRY_CUDA(make_slab_tmap(&mx, px, kF32, Pf, W + 2, m + 2, geom), "osc_tv_ooc: tensor map");
-    MEXCT_TRY_CUDA(make_slab_tmap(&my, py, kF32, Pf, W + 2, m + 2, geom), "osc_tv_ooc: tensor map");
+    MEXCT_TRY_CUDA(make_fp_tmaps(rows, geom, px, py, kF32, W, m, &mx, &my),
+                   "osc_tv_ooc: tensor map");
     for (int v0 = 0; v0 < nv; v0 += kMaxViews) {
       ra->nviews = std::min(kMaxViews, nv - v0);
       ra->view0 = v0;
       for (int i = 0; i < ra->nviews; ++i) ra->trig[i] = trig[v0 + i];
-      MEXCT_TRY_CUDA(launch_fp_slab_sub(geom, *ra, mx, my, px, py, Pf, d_l, epi, st),
+      MEXCT_TRY_CUDA(launch_fp_slab_sub(geom, *ra, mx, my, px, py, fp_layout(rows, W, m, kF32).pitch,
+                                        d_l, epi, st),
                      "osc_tv_ooc: fp");
     }
     return MEXCT_OK;
@@ -393,7 +396,7 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
       mexct_status e = run_slab(io, z0, z1, [&](int bs, const float**) -> mexct_status {
         float* px = Wk[bs];
         float* py = Wk[bs] + pad_half;
-        MEXCT_TRY_CUDA(launch_pad_volume_sub(X[bs], W, m, Pf, false, false, px, py, st, true),
+        MEXCT_TRY_CUDA(launch_pad_volume_sub(rows, X[bs], W, m, false, false, px, py, st, true),
                        "osc_tv_ooc: pad");
         return fp_part(px, py, z0, m, nv, i > 0);
       });
@@ -419,15 +422,15 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
         mexct_status e = run_slab(io, z0, z1, [&](int bs, const float** out) -> mexct_status {
           float* px = Wk[bs];
           float* py = Wk[bs] + pad_half;
-          MEXCT_TRY_CUDA(launch_pad_volume_sub(X[bs], W, m, Pf, false, false, px, py, st, true),
+          MEXCT_TRY_CUDA(launch_pad_volume_sub(rows, X[bs], W, m, false, false, px, py, st, true),
                          "osc_tv_ooc: pad");
           fill_vox(*va, W, H, sad);
           va->zoff = z0;
           va->nzs = m;
           va->nviews = nvu;
           for (int j = 0; j < nvu; ++j) va->trig[j] = tu[j];
-          MEXCT_TRY_CUDA(launch_osc_bp_update(geom, *va, d_rpre, d_rpost, X[bs], kF32, px, py, Pf,
-                                              st),
+          MEXCT_TRY_CUDA(launch_osc_bp_update(geom, *va, d_rpre, d_rpost, X[bs], kF32, px, py,
+                                              fp_layout(rows, W, m, kF32).pitch, st),
                          "osc_tv_ooc: bp/update");
           if (!last) {
             if (mexct_status e2 = fp_part(px, py, z0, m, nvn, i > 0)) return e2;

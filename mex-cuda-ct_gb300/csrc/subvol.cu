@@ -107,26 +107,28 @@ mexct_status fp_sub_impl(mexct_ctx* c, const float* d_slab, int W, int H, int z0
   a->zlo = (float)(rlo - 1);
   a->zhi = (float)(rhi + 1);
   a->accum = accumulate ? 1 : 0;
-  const int Pf = slab_pitch(W);
-  const size_t bytes = (size_t)Pf * (W + 2) * (nz + 2) * sizeof(float);
-  MEXCT_TRY_CUDA(c->padx.ensure_async(bytes, st), "fp_sub: workspace");
-  MEXCT_TRY_CUDA(c->pady.ensure_async(bytes, st), "fp_sub: workspace");
+  a->nall = nP;
+  const bool rows = fp_uses_rows(geom);
+  const FpLayout L = fp_layout(rows, W, nz, kF32);
+  MEXCT_TRY_CUDA(c->padx.ensure_async(L.px, st), "fp_sub: workspace");
+  MEXCT_TRY_CUDA(c->pady.ensure_async(L.py, st), "fp_sub: workspace");
   if (!c->err.p) {
     MEXCT_TRY_CUDA(c->err.ensure(64), "fp_sub: workspace");
     MEXCT_TRY_CUDA(cudaMemset(c->err.p, 0, 64), "fp_sub: workspace");
   }
-  MEXCT_TRY_CUDA(launch_pad_volume_sub(d_slab, W, nz, Pf, z0 > 0, z0 + nz < H,
+  MEXCT_TRY_CUDA(launch_pad_volume_sub(rows, d_slab, W, nz, z0 > 0, z0 + nz < H,
                                        c->padx.as<float>(), c->pady.as<float>(), st),
                  "fp_sub: pad");
   CUtensorMap mx, my;
-  MEXCT_TRY_CUDA(make_slab_tmap(&mx, c->padx.p, kF32, Pf, W + 2, nz + 2, geom), "fp_sub: tensor map");
-  MEXCT_TRY_CUDA(make_slab_tmap(&my, c->pady.p, kF32, Pf, W + 2, nz + 2, geom), "fp_sub: tensor map");
+  MEXCT_TRY_CUDA(make_fp_tmaps(rows, geom, c->padx.p, c->pady.p, kF32, W, nz, &mx, &my),
+                 "fp_sub: tensor map");
   SlabEpi e{nullptr, nullptr, nullptr, nullptr, c->err.as<unsigned>(), c->wait_us};
   for (int v0 = 0; v0 < nP; v0 += kMaxViews) {
     a->nviews = std::min(kMaxViews, nP - v0);
     a->view0 = v0;
     for (int i = 0; i < a->nviews; ++i) trig_of(angles[v0 + i], &a->trig[i]);
-    MEXCT_TRY_CUDA(launch_fp_slab_sub(geom, *a, mx, my, c->padx.p, c->pady.p, Pf, d_sino, e, st),
+    MEXCT_TRY_CUDA(launch_fp_slab_sub(geom, *a, mx, my, c->padx.p, c->pady.p, L.pitch, d_sino,
+                                      e, st),
                    "fp_sub: launch");
   }
   return MEXCT_OK;
@@ -178,9 +180,11 @@ mexct_status bp_sub_impl(mexct_ctx* c, const float* d_rows, int row0, int nrows,
   return MEXCT_OK;
 }
 
-// Device bytes of one FP slab of nz slices (slab + two padded layouts).
+// Device bytes of one FP slab of nz slices (slab + padded layouts; the larger
+// of the geometries').
 size_t fp_slab_bytes(int W, int nz) {
-  return (size_t)W * W * nz * 4 + 2 * (size_t)slab_pitch(W) * (W + 2) * (nz + 2) * 4;
+  const FpLayout s = fp_layout(false, W, nz, kF32);
+  return (size_t)W * W * nz * 4 + std::max(s.px + s.py, rows_bytes(W, nz, kF32));
 }
 
 // Views laid out per BP launch of the out-of-core driver: the layout holds a
