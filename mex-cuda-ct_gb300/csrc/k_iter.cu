@@ -10,9 +10,13 @@
 //   tv_update_kernel gradient recomputed, y = x + scale*g into the other
 //                    buffer of a ping-pong pair.
 // Algorithmic traffic is 12 bytes per voxel per step (read x twice, write y).
+// Whole FP32 descents take tv_fused_kernel instead: one sweep and one gradient
+// per step.  The pair serves FP16 / BF16, the sub-volume sweeps and the
+// allocation-free form (one scratch volume).
 // FP32 volumes whose x extent is a multiple of 4 use tv4_kernel (four x-voxels
 // per thread, 16-byte loads and stores, packed FP32x2 arithmetic): 512^3 step
 // 0.92 -> 0.55 ms, 2.9 TB/s of algorithmic traffic; other volumes tv_sweep.
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
@@ -214,8 +218,8 @@ __global__ void __launch_bounds__(kTvBx * kTvBy) tv_update_kernel(
 // shared by four voxels.  A CTA of 32 x 16 threads covers 128 x 16 columns
 // and owns 124 x 15 of them: the last lane's four columns and the last row
 // give the +x / +y neighbours' terms (the stride of 124 keeps every segment
-// 16-byte aligned).  The norm's per-thread FP32 partial covers its 4 x 32
-// voxels; everything above is FP64 as in tv_norm_kernel.
+// 16-byte aligned).  The norm sums a segment's squares in FP32 and segments as
+// two floats (add_squares); everything above is FP64 as in tv_norm_kernel.
 // ---------------------------------------------------------------------------
 constexpr int kT4Bx = 32, kT4By = 16, kT4Z = 32;
 constexpr int kT4Ox = kT4Bx * 4 - 4, kT4Oy = kT4By - 1;  // 124 x 15 outputs
@@ -236,6 +240,42 @@ __device__ __forceinline__ V4 add4(V4 a, V4 b) { return V4{__fadd2_rn(a.lo, b.lo
 __device__ __forceinline__ V4 mul4(V4 a, V4 b) { return V4{__fmul2_rn(a.lo, b.lo), __fmul2_rn(a.hi, b.hi)}; }
 __device__ __forceinline__ V4 fma4(V4 a, V4 b, V4 c) {
   return V4{__ffma2_rn(a.lo, b.lo, c.lo), __ffma2_rn(a.hi, b.hi, c.hi)};
+}
+
+// 1 / (eps + |(a, b, c)|) of four voxels by the hardware reciprocal square root
+// and reciprocal: |.| = s2 rsqrt(s2).  s2 starts from FLT_MIN (no effect beside
+// eps), so both arguments are normal and the flush-to-zero forms give what
+// rsqrtf and a division of 1 give, without their range tests.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_normal(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ V4 tv_recip(V4 a, V4 b, V4 c) {
+  const float2 tiny = make_float2(1.17549435e-38f, 1.17549435e-38f);
+  const float2 eps = make_float2(1.0e-6f, 1.0e-6f);
+  const V4 s2 = fma4(c, c, fma4(b, b, fma4(a, a, V4{tiny, tiny})));
+  const V4 rs{make_float2(rsqrt_normal(s2.lo.x), rsqrt_normal(s2.lo.y)),
+              make_float2(rsqrt_normal(s2.hi.x), rsqrt_normal(s2.hi.y))};
+  const V4 den = fma4(s2, rs, V4{eps, eps});
+  return V4{make_float2(rcp_normal(den.lo.x), rcp_normal(den.lo.y)),
+            make_float2(rcp_normal(den.hi.x), rcp_normal(den.hi.y))};
+}
+
+// Sum of squares of the four voxels of a segment in FP32, added to a running
+// sum kept as two floats (the rounding of every addition in lo): a thread's
+// sum is good to ~1e-14, so the norm does not depend on which tiles grouped
+// the segments, and the kernels that tile differently give the same step scale.
+__device__ __forceinline__ void add_squares(float4 g, float2& sum) {
+  const float q = fmaf(g.w, g.w, fmaf(g.z, g.z, fmaf(g.y, g.y, g.x * g.x)));
+  const float s = sum.x + q, b = s - sum.x;
+  sum.y += (sum.x - (s - b)) + (q - b);
+  sum.x = s;
 }
 
 // mode 0: ||g||^2 reduction (scale / norm written by the last CTA);
@@ -277,7 +317,7 @@ __global__ void __launch_bounds__(kT4Bx * kT4By, 2) tv4_kernel(
   float xl = (ld_l && z0 < Nz) ? __ldg(v + oc - 1) : 0.f;
   V4 q0p{}, qap{}, xz{};
   float qa_next = 0.f;  // +x neighbour's qa of the previous plane (lane + 1, element 0)
-  float ss = 0.f;
+  float2 ss = make_float2(0.f, 0.f);
 #pragma unroll 1
   for (int p = z0; p <= zend; ++p) {
     // prefetch the next plane
@@ -290,17 +330,10 @@ __global__ void __launch_bounds__(kT4Bx * kT4By, 2) tv4_kernel(
     const float left = __shfl_up_sync(0xffffffffu, xc4.w, 1);
     const V4 xm{make_float2(tx == 0 ? xl : left, xc4.x), make_float2(xc4.y, xc4.z)};
     const V4 a = sub4(xc, xm), b = sub4(xc, xy), cc = sub4(xc, xprev);
-    const V4 s2 = fma4(cc, cc, fma4(b, b, mul4(a, a)));
-    // |(a,b,c)| = s2 * rsqrt(s2) (0 for s2 = 0: the argument is kept >= FLT_MIN,
-    // where eps dominates anyway), r = 1/(eps + |.|), 0 where q does not exist
-    const V4 rs{make_float2(rsqrtf(fmaxf(s2.lo.x, 1.17549435e-38f)), rsqrtf(fmaxf(s2.lo.y, 1.17549435e-38f))),
-                make_float2(rsqrtf(fmaxf(s2.hi.x, 1.17549435e-38f)), rsqrtf(fmaxf(s2.hi.y, 1.17549435e-38f)))};
-    const float2 eps2 = make_float2(1.0e-6f, 1.0e-6f);
-    const V4 den{__fadd2_rn(eps2, __fmul2_rn(s2.lo, rs.lo)), __fadd2_rn(eps2, __fmul2_rn(s2.hi, rs.hi))};
+    // 0 where q does not exist
     const float qm = (incol && gy >= 1 && p >= 1 && p < Nz) ? 1.f : 0.f;
     const float2 qm2 = make_float2(qm, qm);
-    const V4 r{__fmul2_rn(qm2, make_float2(__fdividef(1.0f, den.lo.x), __fdividef(1.0f, den.lo.y))),
-               __fmul2_rn(qm2, make_float2(__fdividef(1.0f, den.hi.x), __fdividef(1.0f, den.hi.y)))};
+    const V4 r = mul4(V4{qm2, qm2}, tv_recip(a, b, cc));
     const V4 q0 = mul4(add4(add4(a, b), cc), r);
     const V4 qa = mul4(a, r), qb = mul4(b, r), qc = mul4(cc, r);
     if (p > z0) {
@@ -313,12 +346,7 @@ __global__ void __launch_bounds__(kT4Bx * kT4By, 2) tv4_kernel(
       const float2 zm2 = make_float2(zm, zm);
       g = V4{__fmul2_rn(__fmul2_rn(g.lo, xmask.lo), zm2), __fmul2_rn(__fmul2_rn(g.hi, xmask.hi), zm2)};
       if (MODE == 0) {
-        if (own) {
-          ss = fmaf(g.lo.x, g.lo.x, ss);
-          ss = fmaf(g.lo.y, g.lo.y, ss);
-          ss = fmaf(g.hi.x, g.hi.x, ss);
-          ss = fmaf(g.hi.y, g.hi.y, ss);
-        }
+        if (own) add_squares(make_float4(g.lo.x, g.lo.y, g.hi.x, g.hi.y), ss);
       } else if (own) {
         const float2 lo = __ffma2_rn(a2, g.lo, xz.lo), hi = __ffma2_rn(a2, g.hi, xz.hi);
         *reinterpret_cast<float4*>(yout + (oc - sz)) = make_float4(lo.x, lo.y, hi.x, hi.y);
@@ -337,7 +365,7 @@ __global__ void __launch_bounds__(kT4Bx * kT4By, 2) tv4_kernel(
     __syncthreads();
   }
   if (MODE == 0) {
-    const double blk = block_sum((double)ss);
+    const double blk = block_sum((double)ss.x + (double)ss.y);
     double total;
     if (finish_partials(blk, partials, counter, &total)) {
       const double m = sqrt(total);
@@ -346,6 +374,317 @@ __global__ void __launch_bounds__(kT4Bx * kT4By, 2) tv4_kernel(
       *scale = (float)(-ce / m);
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// Fused TV steps (FP32).  tv_norm + tv_update evaluate the gradient twice per
+// step.  Here a sweep stores it: step k reads x_k and g_k = g(x_k), forms
+// x_{k+1} = x_k + scale_k g_k on its tile and the tile's halo, and in the same
+// sweep writes x_{k+1}, g_{k+1} = g(x_{k+1}) and its norm: one gradient per
+// step and 16 bytes per voxel instead of two gradients and 12 bytes (the pair
+// was issue-bound at 80 % of the issue slots).  Per voxel the operations are
+// tv4_kernel's, in its order; only the norm's partial sums are grouped by
+// other tiles.
+//
+// A CTA is 8 rows (7 of them its own) of WX warps of 128 columns.  Tiles do not
+// overlap in x: the right neighbour's term crosses warps through shared memory
+// with the +y terms, and past the tile's end its last lane evaluates that one
+// term itself (at 256^3 tv4_kernel's 124-column tiles covered 372 columns and
+// filled 1.4 waves).  Buffers between the steps have rows of a multiple of four
+// voxels (the spare columns hold zeros), so any Nx takes this path: only the
+// first two sweeps read the caller's rows (XVEC: whole and aligned rows).
+// 20 steps, pairs -> fused: 64^3 0.82 -> 0.21 ms, 127^3 0.90 -> 0.30, 256^3
+// 1.99 -> 1.26 (60 us a sweep: 240 MB of DRAM traffic, 3.9 TB/s; loads one
+// plane ahead in 32 warps of 64 registers per SM is what waits, long
+// scoreboard first), 255^2 x 201 2.31 -> 1.28, 384^2 x 300 4.23 -> 3.55,
+// 512^3 10.95 -> 9.99.  Measured and not kept: 1024-thread CTAs over 512
+// columns (384^2 x 300: 4.53 ms), L2 prefetches four planes ahead (1.93 ms at
+// 256^3).
+// ---------------------------------------------------------------------------
+constexpr int kTfRows = 8, kTfOy = kTfRows - 1;
+
+struct TvFused {
+  const float* x;   // x_k: rows of xp voxels
+  const float* g;   // g_k (mode 1)
+  float* y;         // x_{k+1} (mode 1)
+  float* gout;      // g of the sweep's volume
+  int xp, gp;       // row pitch of x; of g, y and gout (a multiple of 4)
+  int Nx, Ny, Nz, zc;
+  float c;
+  const double* cmul;
+  double* partials;
+  unsigned* counter;
+  const float* scale_in;
+  float* scale_out;
+  double* norm;
+};
+
+// mode 0: g and norm of x; mode 1: x + scale g, then g and norm of that.
+// EDGE: several tiles along x (WX = 1; 80 registers instead of 64).
+template <int MODE, int WX, bool XVEC, bool EDGE>
+__global__ void __launch_bounds__(32 * WX * kTfRows, EDGE ? 3 : 4 / WX) tv_fused_kernel(const TvFused A) {
+  constexpr int TX = 32 * WX;
+  __shared__ float4 qbs[2][kTfRows][TX];
+  __shared__ float qas[2][kTfRows][WX + 1];
+  const int tx = threadIdx.x, ty = threadIdx.y, lane = tx & 31, wx = tx >> 5;
+  const int gx0 = blockIdx.x * (4 * TX) + tx * 4, gy = blockIdx.y * kTfOy + ty;
+  const int Nx = A.Nx, Ny = A.Ny, Nz = A.Nz;
+  const int z0 = blockIdx.z * A.zc, zend = min(z0 + A.zc, Nz);
+  const bool incol = gx0 < Nx && gy < Ny;
+  const bool own = incol && (ty < kTfOy || gy == Ny - 1);
+  // the last lane needs a column past the tile
+  const bool rgt = EDGE && lane == 31 && blockIdx.x != gridDim.x - 1;
+  const bool row_int = gy >= 1 && gy < Ny - 1;
+  bool xin[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) xin[e] = row_int && gx0 + e >= 1 && gx0 + e < Nx - 1;
+  const float s = MODE == 1 ? __ldg(A.scale_in) : 0.f;
+  const float2 s2v = make_float2(s, s);
+  // Loads are unconditional, from the nearest place that exists: a column, row
+  // above, left neighbour or plane that does not exist is read by terms that
+  // no interior voxel takes.
+  const int cx = min(gx0, A.gp - 4), cy = min(gy, Ny - 1), cu = max(cy - 1, 0);
+  const int xsz = A.xp * Ny, gsz = A.gp * Ny;
+  const float* px = A.x + cx + (size_t)A.xp * cy;
+  const float* gx = A.g + cx + (size_t)A.gp * cy;
+  const int xup = (cu - cy) * A.xp, gup = (cu - cy) * A.gp, lf = cx > 0 ? -1 : 0;
+  auto ldx = [&](const float* p) {  // four voxels of a row (those past its end are 0)
+    if (XVEC) return __ldg(reinterpret_cast<const float4*>(p));
+    float4 v;
+    v.x = __ldg(p);
+    v.y = cx + 1 < Nx ? __ldg(p + 1) : 0.f;
+    v.z = cx + 2 < Nx ? __ldg(p + 2) : 0.f;
+    v.w = cx + 3 < Nx ? __ldg(p + 3) : 0.f;
+    return v;
+  };
+  auto ldg4 = [&](const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
+  auto step4 = [&](float4 x, float4 g) {  // x + s g
+    V4 r{__ffma2_rn(s2v, make_float2(g.x, g.y), make_float2(x.x, x.y)),
+         __ffma2_rn(s2v, make_float2(g.z, g.w), make_float2(x.z, x.w))};
+    return r;
+  };
+  // raw values of plane p: own segment, the row above, the left neighbour
+  struct Raw {
+    float4 x, xu, g, gu;
+    float xl, gl;            // left of the warp
+    float xr, xru, gr, gru;  // right of the tile, and above that
+  };
+  auto load = [&](int p) {
+    Raw r;
+    const int pc = min(max(p, 0), Nz - 1);
+    const float* xo = px + (size_t)pc * xsz;
+    r.x = ldx(xo);
+    r.xu = ldx(xo + xup);
+    r.xl = lane == 0 ? __ldg(xo + lf) : 0.f;
+    r.xr = r.xru = r.gr = r.gru = 0.f;
+    if (EDGE && rgt) {
+      r.xr = __ldg(xo + 4);
+      r.xru = __ldg(xo + xup + 4);
+    }
+    if (MODE == 1) {
+      const float* go = gx + (size_t)pc * gsz;
+      r.g = ldg4(go);
+      r.gu = ldg4(go + gup);
+      r.gl = lane == 0 ? __ldg(go + lf) : 0.f;
+      if (EDGE && rgt) {
+        r.gr = __ldg(go + 4);
+        r.gru = __ldg(go + gup + 4);
+      }
+    }
+    return r;
+  };
+  V4 prev;
+  float prevr = 0.f;
+  {
+    const size_t pc = max(z0 - 1, 0);
+    const float4 xv = ldx(px + pc * xsz);
+    prev = MODE == 1 ? step4(xv, ldg4(gx + pc * gsz)) : v4(xv);
+    if (EDGE && rgt) {
+      prevr = __ldg(px + pc * xsz + 4);
+      if (MODE == 1) prevr = fmaf(s, __ldg(gx + pc * gsz + 4), prevr);
+    }
+  }
+  Raw cur = load(z0);
+  int og = gx0 + A.gp * gy + z0 * gsz;  // this plane's segment in y and gout
+  V4 q0p{}, qap{};
+  float qa_next = 0.f;
+  float2 ss = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int p = z0; p <= zend; ++p) {
+    const Raw nxt = load(p + 1);
+    const V4 xc = MODE == 1 ? step4(cur.x, cur.g) : v4(cur.x);
+    const V4 xu = MODE == 1 ? step4(cur.xu, cur.gu) : v4(cur.xu);
+    const float xl = MODE == 1 ? fmaf(s, cur.gl, cur.xl) : cur.xl;
+    if (MODE == 1 && own && p < zend)
+      *reinterpret_cast<float4*>(A.y + og) = make_float4(xc.lo.x, xc.lo.y, xc.hi.x, xc.hi.y);
+    const float left = __shfl_up_sync(0xffffffffu, xc.hi.y, 1);
+    const V4 xm{make_float2(lane == 0 ? xl : left, xc.lo.x), make_float2(xc.lo.y, xc.hi.x)};
+    const V4 a = sub4(xc, xm), b = sub4(xc, xu), cc = sub4(xc, prev);
+    const V4 r = tv_recip(a, b, cc);
+    const V4 q0 = mul4(add4(add4(a, b), cc), r);
+    const V4 qa = mul4(a, r), qb = mul4(b, r), qc = mul4(cc, r);
+    if (p > z0) {
+      // g of plane z = p - 1; every term it takes exists where it is interior
+      const int z = p - 1;
+      if (lane == 31) qa_next = qas[z & 1][ty][wx + 1];
+      const float4 qbb = qbs[z & 1][min(ty + 1, kTfRows - 1)][tx];
+      const V4 qan{make_float2(qap.lo.y, qap.hi.x), make_float2(qap.hi.y, qa_next)};
+      const V4 g = sub4(sub4(sub4(q0p, qan), v4(qbb)), qc);
+      float4 gm = make_float4(xin[0] ? g.lo.x : 0.f, xin[1] ? g.lo.y : 0.f,
+                              xin[2] ? g.hi.x : 0.f, xin[3] ? g.hi.y : 0.f);
+      if (z < 1 || z >= Nz - 1) gm = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (own) {
+        add_squares(gm, ss);
+        *reinterpret_cast<float4*>(A.gout + (og - gsz)) = gm;
+      }
+    }
+    qbs[p & 1][ty][tx] = make_float4(qb.lo.x, qb.lo.y, qb.hi.x, qb.hi.y);
+    if (lane == 0) qas[p & 1][ty][wx] = qa.lo.x;
+    qa_next = __shfl_down_sync(0xffffffffu, qa.lo.x, 1);
+    if (EDGE) {  // the term of the first column past the tile, kept for plane p
+      const float xr = MODE == 1 ? fmaf(s, cur.gr, cur.xr) : cur.xr;
+      const float xru = MODE == 1 ? fmaf(s, cur.gru, cur.xru) : cur.xru;
+      const float ar = xr - xc.hi.y, br = xr - xru, cr = xr - prevr;
+      const float sr = fmaf(cr, cr, fmaf(br, br, fmaf(ar, ar, 1.17549435e-38f)));
+      const float qr = ar * rcp_normal(fmaf(sr, rsqrt_normal(sr), 1.0e-6f));
+      if (lane == 31) qas[p & 1][ty][WX] = qr;
+      prevr = xr;
+    }
+    q0p = q0;
+    qap = qa;
+    prev = xc;
+    cur = nxt;
+    og += gsz;
+    __syncthreads();
+  }
+  const double blk = block_sum((double)ss.x + (double)ss.y);
+  double total;
+  if (finish_partials(blk, A.partials, A.counter, &total)) {
+    const double m = sqrt(total);
+    const double ce = A.cmul ? (double)A.c * __ldcg(A.cmul) : (double)A.c;
+    *A.norm = m;
+    *A.scale_out = (float)(-ce / m);
+  }
+}
+
+// out = x + scale g, from rows of xp and gp voxels to the caller's rows of Nx.
+// out may be x.
+__global__ void __launch_bounds__(256) tv_last_kernel(const float* x, int xp,
+                                                      const float* __restrict__ g, int gp,
+                                                      float* out, int Nx, long long rows,
+                                                      const float* __restrict__ scale) {
+  const float s = __ldg(scale);
+  const long long step = (long long)gridDim.x * 8;
+  for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += step)
+    for (int i = threadIdx.x & 31; i < Nx; i += 32)
+      out[r * Nx + i] = fmaf(s, __ldg(g + r * gp + i), x[r * xp + i]);
+}
+
+__global__ void __launch_bounds__(256) tv_last4_kernel(const float4* x,
+                                                       const float4* __restrict__ g, float4* out,
+                                                       long long n,
+                                                       const float* __restrict__ scale) {
+  const float s = __ldg(scale);
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    const float4 a = x[i], b = __ldg(g + i);
+    out[i] = make_float4(fmaf(s, b.x, a.x), fmaf(s, b.y, a.y), fmaf(s, b.z, a.z), fmaf(s, b.w, a.w));
+  }
+}
+
+static int tvf_pitch(int Nx) { return (Nx + 3) & ~3; }
+// Warps along x: one or two for rows of one tile, else tiles of one.
+static int tvf_wx(int Nx) { return Nx > 128 && Nx <= 256 ? 2 : 1; }
+
+// Tiles of a fused sweep.  Slices per CTA: 32 (one slice in 33 is done twice),
+// fewer where the grid would leave SMs idle.
+static dim3 tvf_grid(int Nx, int Ny, int Nz, int* zc) {
+  const int wx = tvf_wx(Nx);
+  const unsigned gx = (Nx + 128 * wx - 1) / (128 * wx);
+  const unsigned gy = std::max(1, (Ny - 1 + kTfOy - 1) / kTfOy);
+  int z = 32;
+  while (z > 4 && 2 * (long long)gx * gy * ((Nz + z - 1) / z) * wx < 7ll * device_sms()) z /= 2;
+  *zc = z;
+  return dim3(gx, gy, (Nz + z - 1) / z);
+}
+
+size_t tv_fused_elems(int Nx, int Ny, int Nz) { return (size_t)tvf_pitch(Nx) * Ny * Nz; }
+
+size_t tv_fused_partials(int Nx, int Ny, int Nz) {
+  int zc;
+  const dim3 g = tvf_grid(Nx, Ny, Nz, &zc);
+  return (size_t)g.x * g.y * g.z;
+}
+
+bool tv_fused_ok(int Nx, int Ny, int Nz) {
+  int zc;
+  const dim3 g = tvf_grid(Nx, Ny, Nz, &zc);
+  return g.y <= 65535 && g.z <= 65535 &&
+         (long long)tvf_pitch(Nx) * Ny * ((long long)Nz + 2) < (1LL << 31);
+}
+
+template <int MODE, bool XVEC>
+static cudaError_t tvf_go(const TvFused& a, dim3 grd, cudaStream_t st) {
+  const int wx = tvf_wx(a.Nx);
+  const dim3 blk(32 * wx, kTfRows);
+  if (wx == 2) tv_fused_kernel<MODE, 2, XVEC, false><<<grd, blk, 0, st>>>(a);
+  else if (grd.x == 1) tv_fused_kernel<MODE, 1, XVEC, false><<<grd, blk, 0, st>>>(a);
+  else tv_fused_kernel<MODE, 1, XVEC, true><<<grd, blk, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_tv_fused(const float* in, float* out, int Nx, int Ny, int Nz, float c,
+                            const double* cmul, int n_steps, float* work[4], double* partials,
+                            unsigned* counter, float* scale2, double* norm, cudaStream_t st) {
+  const int gp = tvf_pitch(Nx);
+  // x_1, x_2, ... alternate between work[0] and work[3] (null: the rows are
+  // whole, x_2, x_4, ... go to out); g_0, g_1, ... between work[1] and work[2]
+  const bool whole = Nx % 4 == 0 && ((uintptr_t)in & 15) == 0 && ((uintptr_t)out & 15) == 0;
+  float* xb[2] = {work[0], whole ? out : work[3]};
+  if (!xb[1]) return cudaErrorInvalidValue;
+  TvFused a{};
+  a.gp = gp;
+  a.Nx = Nx;
+  a.Ny = Ny;
+  a.Nz = Nz;
+  const dim3 grd = tvf_grid(Nx, Ny, Nz, &a.zc);
+  a.c = c;
+  a.cmul = cmul;
+  a.partials = partials;
+  a.counter = counter;
+  a.norm = norm;
+  const float* x = in;
+  int xp = Nx;
+  for (int k = 0; k < n_steps; ++k) {  // g_k, from x_{k-1} and g_{k-1} for k > 0
+    a.x = x;
+    a.xp = xp;
+    a.gout = work[1 + (k & 1)];
+    a.scale_out = scale2 + (k & 1);
+    const bool vec = xp % 4 == 0 && ((uintptr_t)x & 15) == 0;
+    cudaError_t e;
+    if (k == 0) {
+      e = vec ? tvf_go<0, true>(a, grd, st) : tvf_go<0, false>(a, grd, st);
+    } else {
+      a.g = work[1 + ((k - 1) & 1)];
+      a.scale_in = scale2 + ((k - 1) & 1);
+      a.y = xb[(k - 1) & 1];
+      e = vec ? tvf_go<1, true>(a, grd, st) : tvf_go<1, false>(a, grd, st);
+      x = a.y;
+      xp = gp;
+    }
+    if (e != cudaSuccess) return e;
+  }
+  const float* g = work[1 + ((n_steps - 1) & 1)];
+  const float* scale = scale2 + ((n_steps - 1) & 1);
+  const int ctas = device_sms() * 8;
+  if (xp == Nx && gp == Nx && (((uintptr_t)x | (uintptr_t)out) & 15) == 0) {
+    tv_last4_kernel<<<ctas, 256, 0, st>>>(reinterpret_cast<const float4*>(x),
+                                          reinterpret_cast<const float4*>(g),
+                                          reinterpret_cast<float4*>(out),
+                                          (long long)Nx / 4 * Ny * Nz, scale);
+  } else {
+    tv_last_kernel<<<ctas, 256, 0, st>>>(x, xp, g, gp, out, Nx, (long long)Ny * Nz, scale);
+  }
+  return cudaGetLastError();
 }
 
 static bool tv4_ok(const void* x, const void* y, int xt, int Nx, int Ny, int Nz) {

@@ -309,6 +309,19 @@ cudaError_t launch_tv_update(const void* x, void* y, int x_type, int Nx,
                              int Ny, int Nz, const float* scale,
                              cudaStream_t st);
 
+// n_steps >= 1 whole TV steps of an FP32 volume, one gradient per step: in ->
+// out (which may be the same).  work: buffers of tv_fused_elems floats each
+// (16-byte aligned); [0] x, [1] and [2] gradients, [3] x again, needed only
+// when Nx % 4 != 0 or in / out are not 16-byte aligned (else may be null).
+// scale2: two floats; partials: tv_fused_partials doubles; counter must be 0.
+// c is multiplied by *cmul (device) when cmul is not null.
+bool tv_fused_ok(int Nx, int Ny, int Nz);
+size_t tv_fused_elems(int Nx, int Ny, int Nz);
+size_t tv_fused_partials(int Nx, int Ny, int Nz);
+cudaError_t launch_tv_fused(const float* in, float* out, int Nx, int Ny, int Nz, float c,
+                            const double* cmul, int n_steps, float* work[4], double* partials,
+                            unsigned* counter, float* scale2, double* norm, cudaStream_t st);
+
 // Sum of squared differences in FP64 (OSC_TV_recon.m:65-67), deterministic.
 cudaError_t launch_ssd(const void* a, const void* b, int dtype, long long n,
                        int zero_first, double* partials, unsigned* counter,

@@ -689,7 +689,31 @@ mexct_status tv_dev_impl(mexct_ctx* c, const void* d_in, int t, int Nx,
       MEXCT_TRY_CUDA(cudaMemcpyAsync(d_out, d_in, bytes, cudaMemcpyDeviceToDevice, st), "tvmin3d: copy");
     return MEXCT_OK;
   }
-  MEXCT_TRY_CUDA(ensure_reduction(c, tv_partials_needed(Nx, Ny, Nz)), "tvmin3d: workspace");
+  MEXCT_TRY_CUDA(ensure_reduction(c, std::max(tv_partials_needed(Nx, Ny, Nz),
+                                              tv_fused_partials(Nx, Ny, Nz))),
+                 "tvmin3d: workspace");
+  if (t == kF32 && tv_fused_ok(Nx, Ny, Nz)) {
+    // one gradient per step; its three or four buffers may not fit where the
+    // pair of sweeps below (one buffer) does
+    const bool whole = Nx % 4 == 0 && (((uintptr_t)d_in | (uintptr_t)d_out) & 15) == 0;
+    const size_t wb = tv_fused_elems(Nx, Ny, Nz) * sizeof(float);
+    cudaError_t e = cudaSuccess;
+    for (Buf* b : {&c->r1, &c->r2, &c->r3, &c->tvx})
+      if (e == cudaSuccess && (b != &c->tvx || !whole)) e = b->ensure(wb);
+    if (e == cudaSuccess) {
+      float* work[4] = {c->r1.as<float>(), c->r2.as<float>(), c->r3.as<float>(),
+                        whole ? nullptr : c->tvx.as<float>()};
+      MEXCT_TRY_CUDA(launch_tv_fused((const float*)d_in, (float*)d_out, Nx, Ny, Nz, cval, nullptr,
+                                     n_steps, work, c->red.as<double>(), c->cnt.as<unsigned>(),
+                                     c->scal.as<float>(),
+                                     reinterpret_cast<double*>(c->scal.as<char>() + 8), st),
+                     "tvmin3d: steps");
+      return MEXCT_OK;
+    }
+    if (e != cudaErrorMemoryAllocation) return cuda_err(e, "tvmin3d: workspace");
+    cudaGetLastError();
+    for (Buf* b : {&c->r2, &c->r3, &c->tvx}) b->release_synced();
+  }
   MEXCT_TRY_CUDA(c->r1.ensure(bytes), "tvmin3d: workspace");
   const void* src = d_in;
   if (d_in == d_out && (n_steps % 2) == 1) {
