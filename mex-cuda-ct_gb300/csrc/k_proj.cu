@@ -989,6 +989,12 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
   const size_t base = (size_t)iy * A.W + ix;
   const size_t sz = (size_t)A.W * A.W;
   const size_t Ps = (size_t)A.W + 2;
+  // parallel / fan: the FP's z-fastest layout (columns of pitch Pf, a multiple
+  // of four as zl is): a column's FP32 slices in one store
+  constexpr bool rows = GEOM < 2 && !DET;
+  TM* const col = rows && padx ? padx + ((size_t)(iy + 1) * Ps + (ix + 1)) * Pf + zl : nullptr;
+  const bool whole = rows && std::is_same<TM, float>::value && ZC == 4 && zl + ZC <= A.nzs;
+  float4 four = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int j = 0; j < ZC; ++j) {
     const int z = zl + j;
@@ -997,9 +1003,9 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
       const float f = ldp(o);
       const float m = fmaxf(f + (f * num[j] / den[j]), 0.f);
       stf(o, m);
-      if (GEOM < 2 && !DET) {
-        // the parallel / fan FP's z-fastest layout (columns of pitch Pf)
-        if (padx) stf(padx + ((size_t)(iy + 1) * Ps + (ix + 1)) * Pf + z, m);
+      if (rows) {
+        if (whole) (&four.x)[j & 3] = m;
+        else if (col) stf(col + j, m);
       } else if (padx) {
         // the slab FP's padded layouts: x-fastest and y-fastest, frame of one
         const size_t zp = (size_t)(z + 1) * Ps;
@@ -1008,6 +1014,7 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
       }
     }
   }
+  if (rows && whole && col) *reinterpret_cast<float4*>(col) = four;
 }
 
 cudaError_t launch_osc_bp_update_det(int geom, const VoxArgs& a, const float* rpre,

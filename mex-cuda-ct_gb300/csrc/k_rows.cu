@@ -196,16 +196,16 @@ __device__ __noinline__ float4 rows_slow(const TV* vol, const RowsRay r, bool xd
 
 // EPI 0: line integrals (accum: added to the output); 1: OSC residuals; 2:
 // objective partials.  V views per CTA, NB staged planes (2: two CTAs per SM;
-// 4: one CTA per SM, for grids that leave it alone there).  SP = 4: a cluster
-// of four CTAs shares the tile, a quarter of the planes each; the quarters'
-// sums are added in order from the CTAs' shared memory, one of a warp's four
-// rays per CTA.
+// 4: one CTA per SM, for grids that leave it alone there).  SP = 4 or 8: a
+// cluster of CTAs shares the tile, a part of the planes each; the parts' sums
+// are added in order from the CTAs' shared memory, one of a warp's four rays
+// (or half of its slices) per CTA.
 template <int EPI, typename TV, typename TO, int V, int NB, int SP>
 __global__ void __launch_bounds__(kRThreads, 2) fp_rows_kernel(
     const __grid_constant__ RayArgs A, const int geom, const __grid_constant__ CUtensorMap tmx,
     const __grid_constant__ CUtensorMap tmy, const TV* __restrict__ vol, int Ph,
     TO* __restrict__ out, const SlabEpi E) {
-  static_assert(SP == 1 || (SP == 4 && V == 1 && EPI != 2), "a cluster takes one view");
+  static_assert(SP == 1 || ((SP == 4 || SP == 8) && V == 1 && EPI != 2), "a cluster takes one view");
   constexpr int NG = kRU / 4, PG = 8 / V;  // ray groups; planes whose weights are made at once
   static_assert(NG == kRThreads / 32, "a warp per four rays");
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -214,6 +214,10 @@ __global__ void __launch_bounds__(kRThreads, 2) fp_rows_kernel(
   const int tid = threadIdx.x, lane = tid & 31, g = tid >> 5;
   const int nvg = (A.nviews + V - 1) / V, tiles_u = (A.det_w + kRU - 1) / kRU;
   const int rank = SP > 1 ? (int)(blockIdx.x % SP) : 0, job = (int)(blockIdx.x / SP);
+  // the ray of each warp's four and the slices of each lane's four that this
+  // CTA finishes
+  constexpr int NZ = SP == 8 ? 2 : 4;
+  const int ray = SP == 8 ? rank >> 1 : rank, zb = SP == 8 ? 2 * (rank & 1) : 0;
   const int vg = job % nvg, tile = (job / nvg) % tiles_u, chunk = (job / nvg) / tiles_u;
   const int u0 = tile * kRU, v0 = vg * V, nv = min(V, A.nviews - v0);
   const int Ps = A.S + 2;
@@ -474,10 +478,11 @@ __global__ void __launch_bounds__(kRThreads, 2) fp_rows_kernel(
       for (int z = 0; z < 4; ++z) part[(4 * i + z) * kRThreads + tid] = q[z];
     }
     cluster_sync();
-    float q[4];
+    float q[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int z = 0; z < 4; ++z) {
-      const float* p = part + (4 * rank + z) * kRThreads + tid;
+      if (z < zb || z >= zb + NZ) continue;
+      const float* p = part + (4 * ray + z) * kRThreads + tid;
       q[z] = cluster_ld(p, 0);
 #pragma unroll
       for (int c = 1; c < SP; ++c) q[z] += cluster_ld(p, c);
@@ -486,7 +491,7 @@ __global__ void __launch_bounds__(kRThreads, 2) fp_rows_kernel(
     acc[0][0][0] = make_float2(q[0], q[1]);
     acc[0][0][1] = make_float2(q[2], q[3]);
     const Trig t = A.trig[v0];
-    redo(acc[0][0], S.ray[0][4 * g + rank], fabsf(t.c) >= fabsf(t.s));
+    redo(acc[0][0], S.ray[0][4 * g + ray], fabsf(t.c) >= fabsf(t.s));
   }
 
   constexpr int NI = SP > 1 ? 1 : 4;  // rays of this thread's warp in each view
@@ -495,10 +500,12 @@ __global__ void __launch_bounds__(kRThreads, 2) fp_rows_kernel(
   for (int r = 0; r < V; ++r) {
     if (r >= nv) continue;
     const long long gv = A.view0 + (long long)(v0 + r) * A.vstride;
-    const int ix0 = u0 + 4 * g + (SP > 1 ? rank : 0);
+    const int ix0 = u0 + 4 * g + (SP > 1 ? ray : 0);
     // detector row = slice of the whole volume
     const size_t gi0 = (size_t)gv * A.P + (size_t)(z0 + A.zoff) * A.det_w + ix0;
-    auto valid = [&](int z, int i) { return z0 + z < A.zrows - 2 && ix0 + i < A.det_w; };
+    auto valid = [&](int z, int i) {
+      return z0 + z < A.zrows - 2 && ix0 + i < A.det_w && z >= zb && z < zb + NZ;
+    };
     float pre[EPI ? 4 : 1][NI], post[EPI ? 4 : 1][NI];
     if constexpr (EPI != 0) {  // all counts before the first store
 #pragma unroll
@@ -580,12 +587,14 @@ long long rows_ctas(const RayArgs& a, int v) {
          ((a.zrows - 2 + kRZ - 1) / kRZ);
 }
 
-// Whether a cluster of four shares each tile's planes: calls of few views,
+// CTAs that share each tile's planes as a cluster: four for calls of few views,
 // whose CTAs would leave SMs idle (an OSC subset: 84^2 x 76, 25 views per
-// subset, an iteration 568 us without, 356 with).  The rule does not look at
+// subset, an iteration of 5 subsets 568 us without, 350 with), eight where that
+// still leaves them idle (64^2 x 40, 3 views, 12 subsets: 366 -> 286 us).  The rule does not look at
 // the slices, so a slab of a volume is summed as the whole volume is.
-bool rows_split(const RayArgs& a) {
-  return (long long)std::max(a.nall, a.nviews) * ((a.det_w + kRU - 1) / kRU) <= device_sms();
+int rows_split(const RayArgs& a) {
+  const long long n = (long long)std::max(a.nall, a.nviews) * ((a.det_w + kRU - 1) / kRU);
+  return 8 * n <= device_sms() ? 8 : n <= device_sms() ? 4 : 1;
 }
 
 // Views per CTA: four or two where the CTAs still fill the GPU and their
@@ -658,14 +667,16 @@ cudaError_t rows_launch(int geom, const RayArgs& a, const CUtensorMap& mx, const
     for (cudaError_t err : {GO(1, 2, 1, true), GO(2, 2, 1, true), GO(4, 2, 1, true)})
       if (err != cudaSuccess) return err;
     if constexpr (EPI != 2)
-      for (cudaError_t err : {GO(1, 2, 4, true), GO(1, 4, 4, true)})
+      for (cudaError_t err : {GO(1, 2, 4, true), GO(1, 4, 4, true), GO(1, 4, 8, true)})
         if (err != cudaSuccess) return err;
     return cudaSuccess;
   }
   // (the objective's partials have room for one CTA per tile)
-  if constexpr (EPI != 2)
-    if (rows_split(a))
-      return 4 * rows_ctas(a, 1) > device_sms() ? GO(1, 2, 4, false) : GO(1, 4, 4, false);
+  if constexpr (EPI != 2) {
+    const int sp = rows_split(a);
+    if (sp == 8) return GO(1, 4, 8, false);
+    if (sp == 4) return 4 * rows_ctas(a, 1) > device_sms() ? GO(1, 2, 4, false) : GO(1, 4, 4, false);
+  }
   const int v = rows_views(geom, a);
   return v == 4 ? GO(4, 2, 1, false) : v == 2 ? GO(2, 2, 1, false) : GO(1, 2, 1, false);
 #undef GO
