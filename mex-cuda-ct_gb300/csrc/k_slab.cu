@@ -1197,7 +1197,17 @@ static cudaError_t slab_go(const RayArgs& a, const CUtensorMap& mx, const CUtens
   }
   if (a.nviews <= 0) return cudaSuccess;
   const int tiles = ((a.det_w + 31) / 32) * ((a.det_h + 7) / 8);
-  const bool pair = GEOM != 3 && slab_pair_views(a);
+  bool pair = GEOM != 3 && slab_pair_views(a);
+  if (pair) {
+    // A small grid's last wave decides: two views per CTA halve the CTAs, so 64^3
+    // x 90 views (720 CTAs on 608 places) took two waves of double work, 95 us,
+    // where one view per CTA takes three of single work.  Pairs save ~2 %
+    // otherwise; per ray the sums are the same bits.
+    const long long places = (long long)kSlabCtas * device_sms();
+    const long long w2 = ((long long)((a.nviews + 1) / 2) * tiles + places - 1) / places;
+    const long long w1 = ((long long)a.nviews * tiles + places - 1) / places;
+    if (w2 <= 4 && w1 < 2 * w2) pair = false;
+  }
   dim3 blk(32, 8), grd(pair ? (a.nviews + 1) / 2 : a.nviews, tiles);
   if (pair)
     k2<<<grd, blk, smem, st>>>(a, mx, my, (const TV*)px, (const TV*)py, Pf, (TO*)out, e);
