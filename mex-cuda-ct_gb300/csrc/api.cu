@@ -133,6 +133,15 @@ void trig_of(float beta, Trig* t) {
   t->c = (float)std::cos((double)beta);
 }
 
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cs != cudaStreamCaptureStatusNone;
+}
+
 mexct_ctx* resolve(mexct_ctx* ctx) {
   if (ctx) return ctx;
   int dev = 0;
@@ -299,6 +308,7 @@ mexct_status mexct_ctx_destroy(mexct_ctx* c) {
       if (ev) cudaEventDestroy(ev);
     cudaStreamDestroy(c->copy_stream);
   }
+  if (c->gpair_ev) cudaEventDestroy(c->gpair_ev);
   cudaStreamDestroy(c->stream);
   cudaSetDevice(prev);
   delete c;

@@ -53,6 +53,9 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Whether st is being captured (an unknown state counts as captured).
+bool capturing(cudaStream_t st);
+
 // One entry of a context's launch-shape table.
 struct TuneEntry {
   mexct_shape shape;
@@ -85,6 +88,8 @@ struct mexct_ctx {
   mexct::Buf spad;   // padded sinogram views for BP
   mexct::Buf bpart;  // BP view-block partial sums
   mexct::Buf subs;   // one sub-ray sinogram of a super-sampled FP
+  mexct::Buf gpair;  // general3D BP: pair buffers, and the end of their last use
+  cudaEvent_t gpair_ev = nullptr;
   mexct::Buf tvx;    // TV: a second volume between steps (rows that are not whole)
   // Launch shapes: MEXCT_TUNE_* mode and the per-class table.
   int tune_mode = MEXCT_TUNE_HEURISTIC;
@@ -116,7 +121,7 @@ struct mexct_ctx {
 
   std::vector<mexct::Buf*> all_bufs() {
     return {&in, &in2, &in3, &out, &volT, &r1, &r2, &r3, &tabs, &red, &cnt, &scal,
-            &padx, &pady, &err, &spad, &bpart, &subs, &tvx};
+            &padx, &pady, &err, &spad, &bpart, &subs, &tvx, &gpair};
   }
 };
 

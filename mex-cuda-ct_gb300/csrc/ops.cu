@@ -480,14 +480,34 @@ mexct_status g3d_bp_dev_impl(mexct_ctx* c, const float* d_sino, int W, int H,
   if (bad_dims(S, Z) || bad_dims(W, H)) return set_err(MEXCT_ERR_ARG, "g3d_bp: bad dims");
   if (nP < 0) return set_err(MEXCT_ERR_ARG, "g3d_bp: bad view count %d", nP);
   if (!c) return MEXCT_OK;  // validate only
-  MEXCT_TRY_CUDA(cudaMemsetAsync(d_vol, 0, (size_t)S * S * Z * sizeof(float), st), "g3d_bp: zero");
+  const size_t N = (size_t)S * S * Z;
+  // Pair buffers where the rays pay for them and they fit.  A call may follow
+  // one on another stream: it waits for the end of the buffers' last use.  A
+  // captured call, whose graph would keep their address, needs none.
+  bool pairs = g3d_bp_pairs(S, Z, (long long)W * H * nP) && !capturing(st);
+  if (pairs) {
+    if (!c->gpair_ev)
+      MEXCT_TRY_CUDA(cudaEventCreateWithFlags(&c->gpair_ev, cudaEventDisableTiming), "g3d_bp: event");
+    MEXCT_TRY_CUDA(cudaStreamWaitEvent(st, c->gpair_ev, 0), "g3d_bp: wait");
+    const cudaError_t e = c->gpair.ensure_async(4 * N * sizeof(float), st);
+    if (e == cudaErrorMemoryAllocation) pairs = false;
+    else if (e != cudaSuccess) return cuda_err(e, "g3d_bp: workspace");
+  }
+  float* acc = pairs ? c->gpair.as<float>() : d_vol;
+  MEXCT_TRY_CUDA(cudaMemsetAsync(acc, 0, (pairs ? 4 : 1) * N * sizeof(float), st), "g3d_bp: zero");
   std::unique_ptr<RayArgs> a(new RayArgs);
   fill_g3d(*a, S, Z, W, H, per_view ? 1 : 0);
   for (int v0 = 0; v0 < nP; v0 += kMaxViews) {
     a->nviews = std::min(kMaxViews, nP - v0);
     a->view0 = v0;
     for (int i = 0; i < a->nviews; ++i) trig_of(angles[v0 + i], &a->trig[i]);
-    MEXCT_TRY_CUDA(launch_g3d_bp(*a, d_sino, d_pts, d_vol, st), "g3d_bp: launch");
+    MEXCT_TRY_CUDA(pairs ? launch_g3d_bp_pairs(*a, d_sino, d_pts, acc, st)
+                         : launch_g3d_bp(*a, d_sino, d_pts, acc, st),
+                   "g3d_bp: launch");
+  }
+  if (pairs) {
+    MEXCT_TRY_CUDA(launch_g3d_bp_fold(acc, S, Z, d_vol, st), "g3d_bp: fold");
+    MEXCT_TRY_CUDA(cudaEventRecord(c->gpair_ev, st), "g3d_bp: event");
   }
   return MEXCT_OK;
 }

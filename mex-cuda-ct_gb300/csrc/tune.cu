@@ -71,15 +71,6 @@ mexct_shape default_shape(const mexct_ctx* c, int op, int W, int H, int nP) {
   return fixed_shape();
 }
 
-bool capturing(cudaStream_t st) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
-    cudaGetLastError();
-    return true;  // unknown: do not time
-  }
-  return cs != cudaStreamCaptureStatusNone;
-}
-
 // Best of the timed runs of fn() on st after one untimed run, in ms.  Short
 // calls are repeated inside each timed run (about 2 ms of work per run) so
 // launch jitter does not pick the shape.
