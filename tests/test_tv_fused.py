@@ -48,3 +48,24 @@ def test_in_place_and_unaligned_equal_out_of_place(cuda, steps, Nx):
     out = torch.empty(vol.numel() + 1, device="cuda")[1:].view(vol.shape)
     ops.tvmin3d_dev(off, 0.05, steps, out=out)
     assert torch.equal(own, ref) and torch.equal(out, ref)
+
+
+def test_captured_call_matches(cuda):
+    """A captured call allocates nothing: it takes the pair of sweeps, and replays."""
+    import torch
+    import mexct
+
+    vol = torch.from_numpy(np.random.default_rng(8).uniform(0, 1, (20, 33, 44)).astype(np.float32)).cuda()
+    out = torch.empty_like(vol)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    mexct.ops.tvmin3d_dev(vol, 0.05, 3, out=out, stream=st)
+    st.synchronize()
+    want = out.clone()
+    out.zero_()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        mexct.ops.tvmin3d_dev(vol, 0.05, 3, out=out, stream=st)
+    g.replay()
+    torch.cuda.synchronize()
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 1e-5
