@@ -1117,8 +1117,12 @@ __global__ void __launch_bounds__(256) prefilter_tiled_kernel(
 // through shared memory for 3 radices.  The zero half of the padded row
 // (W <= N / 2) is never loaded, and only the first half is transformed back.
 // Rows move through memory once: 8 bytes per pixel.  384^2 x 512 views, cone,
-// Hamming: 2.47 -> 0.70 ms (0.87 TB/s: the passes'
-// arithmetic and exchanges, not the memory, bound it); 3 CTAs of 80 registers per SM.
+// Hamming: 2.47 -> 0.49 ms (1.24 TB/s: issue slots 70 % and the shared / L1 data
+// path 61 %, not the memory, bound it); 3 CTAs of 80 registers per SM.  With so
+// few warps the order of the loads counts: tables laid out so that a warp reads
+// neighbours took it from 0.70 to 0.63 ms (the spectrum, 64 bytes apart, had
+// cost as many L1 wavefronts as all exchanges), a row's loads all before its
+// arithmetic and table loads before the barriers to 0.49.
 //
 // The filter all but removes a smooth row, so a transform's rounding (relative
 // to the row) would stand out against the output: 2.2e-6 of it at 384 columns,
@@ -1202,16 +1206,21 @@ __device__ __forceinline__ void dft(float2* v) {
   }
 }
 
-// v[k] *= exp(-+2 pi i k f / N) for k < R: the powers 1, 2, 4, 8 from the
-// table, the others as products of those (loading every power took 745 us
-// where this takes 625 at 384^2 x 512).
+// v[k] *= w^k for k < R: the powers 1, 2, 4, 8 of w from the table, rows of
+// `pitch` elements so that a warp reads neighbours, the others as products of
+// those (loading every power took 745 us where this took 625 at 384^2 x 512).
+template <int R>
+__device__ __forceinline__ void twiddle_load(float2* w, const float2* __restrict__ tw, int pitch) {
+#pragma unroll
+  for (int k = 0; k < (R > 8 ? 4 : R > 4 ? 3 : 2); ++k) w[k] = __ldg(tw + k * pitch);
+}
 template <int R, bool INV>
-__device__ __forceinline__ void twiddle(float2* v, const float2* __restrict__ tw, int f) {
+__device__ __forceinline__ void twiddle(float2* v, const float2* w) {
   float2 p[R];
-  p[1] = c_conj_if<INV>(__ldg(tw + f));
-  p[2] = c_conj_if<INV>(__ldg(tw + 2 * f));
-  if constexpr (R > 4) p[4] = c_conj_if<INV>(__ldg(tw + 4 * f));
-  if constexpr (R > 8) p[8] = c_conj_if<INV>(__ldg(tw + 8 * f));
+  p[1] = c_conj_if<INV>(w[0]);
+  p[2] = c_conj_if<INV>(w[1]);
+  if constexpr (R > 4) p[4] = c_conj_if<INV>(w[2]);
+  if constexpr (R > 8) p[8] = c_conj_if<INV>(w[3]);
 #pragma unroll
   for (int k = 1; k < R; ++k) {
     if (k > 8) p[k] = c_mul(p[8], p[k - 8]);
@@ -1226,13 +1235,10 @@ __device__ __forceinline__ int fft_slot(int i) { return i + (i >> 3); }
 
 // Weighted input sample as prefilter_input, the cosine weight by a reciprocal
 // square root with one Newton step.
-__device__ __forceinline__ float prefilter_fast_input(const FiltArgs& A,
-                                                      const float* __restrict__ sino,
-                                                      const float* __restrict__ pre, size_t gi,
-                                                      int v, int u, float pk) {
-  float s = __ldg(sino + gi);
+__device__ __forceinline__ float prefilter_fast_input(const FiltArgs& A, float s, float pre, int v,
+                                                      int u, float pk) {
   if (A.log_input) {
-    s = -logf(s / __ldg(pre + gi));
+    s = -logf(s / pre);
     if (!isfinite(s)) s = 0.f;
   }
   if (A.geom != 0) {
@@ -1260,7 +1266,7 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   __shared__ float2 psum[NF * NWF], edge[8 * NF * NWF];
   // after the spatial kernel: the differences' spectrum and the twiddles
   const float2* spec = reinterpret_cast<const float2*>(kern + N);
-  const float2* tw = spec + N;
+  const float2 *tw1 = spec + N, *tw2 = tw1 + 4 * TF;
   const int n = threadIdx.x % TF, q = threadIdx.x / TF;
   float2* x = sm + q * (N + N / 8);
   const int W = A.W, H = A.H, hp = (H + 1) >> 1;
@@ -1278,14 +1284,28 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   float2 e[16];
   bool b0 = false, b1 = false;
   {
+    // all loads first, the lower row's twice where the upper is missing
+    float2 raw[8], r0[8];
+    float pk[8];
+    const size_t up = two ? W : 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int u = n + j * TF;
+      raw[j] = r0[j] = make_float2(0.f, 0.f);
+      pk[j] = 0.f;
+      if (live && u < W) {
+        raw[j] = make_float2(__ldg(sino + row0 + u), __ldg(sino + row0 + up + u));
+        if (A.log_input) r0[j] = make_float2(__ldg(pre + row0 + u), __ldg(pre + row0 + up + u));
+        pk[j] = __ldg(parker + (size_t)view * W + u);
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int u = n + j * TF;
       float2 s = make_float2(0.f, 0.f);
       if (live && u < W) {
-        const float pk = __ldg(parker + (size_t)view * W + u);
-        s.x = prefilter_fast_input(A, sino, pre, row0 + u, v0, u, pk);
-        if (two) s.y = prefilter_fast_input(A, sino, pre, row0 + W + u, v0 + 1, u, pk);
+        s.x = prefilter_fast_input(A, raw[j].x, r0[j].x, v0, u, pk[j]);
+        if (two) s.y = prefilter_fast_input(A, raw[j].y, r0[j].y, v0 + 1, u, pk[j]);
       }
       b0 |= !(fabsf(s.x) <= 1.0e30f);
       b1 |= !(fabsf(s.y) <= 1.0e30f);
@@ -1337,26 +1357,34 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
     }
   }
   // radix R1, stride TF
+  float2 w1[4], w2[4];
+  twiddle_load<R1>(w1, tw1 + n, TF);
   dft<R1, false>(e);
-  twiddle<R1, false>(e, tw, n);
+  twiddle<R1, false>(e, w1);
 #pragma unroll
   for (int j = 0; j < 16; ++j) x[fft_slot(n + j * TF)] = e[j];
+  // table loads go out before the barriers they would wait behind
+  const int t = n % R3;  // (n + i TF) % R3
+  if constexpr (R3 > 1) twiddle_load<R2>(w2, tw2 + t, R3);
   __syncthreads();
   if constexpr (R3 > 1) {  // radix R2, stride R3
 #pragma unroll
     for (int i = 0; i < 16 / R2; ++i) {
-      const int b = n + i * TF, t = b % R3, base = (b / R3) * (R2 * R3) + t;
+      const int base = ((n + i * TF) / R3) * (R2 * R3) + t;
 #pragma unroll
       for (int j = 0; j < R2; ++j) e[j] = x[fft_slot(base + j * R3)];
       dft<R2, false>(e);
-      twiddle<R2, false>(e, tw, t * R1);
+      twiddle<R2, false>(e, w2);
 #pragma unroll
       for (int j = 0; j < R2; ++j) x[fft_slot(base + j * R3)] = e[j];
     }
-    __syncthreads();
   }
   {  // last radix, filter, first inverse radix
     constexpr int RL = R3 > 1 ? R3 : R2;
+    float2 sp[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sp[i] = __ldg(spec + i % RL * (N / RL) + n + i / RL * TF);
+    if constexpr (R3 > 1) __syncthreads();
 #pragma unroll
     for (int i = 0; i < 16 / RL; ++i) {
       const int base = (n + i * TF) * RL;
@@ -1371,29 +1399,32 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
         if (bad1) e[0].y = 0.f;
       }
 #pragma unroll
-      for (int j = 0; j < RL; ++j) e[j] = c_mul(e[j], __ldg(spec + base + j));
+      for (int j = 0; j < RL; ++j) e[j] = c_mul(e[j], sp[i * RL + j]);
       dft<RL, true>(e);
 #pragma unroll
       for (int j = 0; j < RL; ++j) x[fft_slot(base + j)] = e[j];
     }
+    if constexpr (R3 > 1) twiddle_load<R2>(w2, tw2 + t, R3);
+    else twiddle_load<R1>(w1, tw1 + n, TF);
     __syncthreads();
   }
   if constexpr (R3 > 1) {
 #pragma unroll
     for (int i = 0; i < 16 / R2; ++i) {
-      const int b = n + i * TF, t = b % R3, base = (b / R3) * (R2 * R3) + t;
+      const int base = ((n + i * TF) / R3) * (R2 * R3) + t;
 #pragma unroll
       for (int j = 0; j < R2; ++j) e[j] = x[fft_slot(base + j * R3)];
-      twiddle<R2, true>(e, tw, t * R1);
+      twiddle<R2, true>(e, w2);
       dft<R2, true>(e);
 #pragma unroll
       for (int j = 0; j < R2; ++j) x[fft_slot(base + j * R3)] = e[j];
     }
+    twiddle_load<R1>(w1, tw1 + n, TF);
     __syncthreads();
   }
 #pragma unroll
   for (int j = 0; j < 16; ++j) e[j] = x[fft_slot(n + j * TF)];
-  twiddle<R1, true>(e, tw, n);
+  twiddle<R1, true>(e, w1);
   dft<R1, true>(e);
   const float db = live ? __ldg(dbeta + view) : 0.f;
 #pragma unroll

@@ -769,9 +769,12 @@ int filter_order(int W) {
 // out: the spatial kernel (order floats); where the FFT form serves the order
 // R1 R2 R3, followed by two complex tables of `order` elements: the spectrum
 // of the filter on a row's differences, H / (order (1 - exp(-i w))) (element 0:
-// H[0] / order, for the row's sum), in digit-reversed order (position
-// (k1 R2 + k2) R3 + k3 holds frequency k1 + R1 k2 + R1 R2 k3), and the
-// twiddles exp(-2 pi i k / order).
+// H[0] / order, for the row's sum), and the twiddles.  The last radix R of the
+// transform leaves frequency k1 + R1 k2 + R1 R2 k3 at position (k1 R2 + k2) R3
+// + k3 = m R + j; it is stored at j order / R + m, for the threads of
+// neighbouring m read it together.  Twiddles: exp(-2 pi i 2^k n / order) at
+// k order / R1 + n (n < order / R1), then, with a third radix, exp(-2 pi i 2^k
+// n R1 / order) at k R3 + n (n < R3), for k < 4.
 void filter_kernel(int W, int filter, double d, std::vector<float>& out) {
   const double pi = 3.14159265358979323846;
   const int order = filter_order(W), half = order / 2;
@@ -815,18 +818,25 @@ void filter_kernel(int W, int filter, double d, std::vector<float>& out) {
   out.resize((size_t)5 * order);
   float* spec = out.data() + order;
   float* tw = spec + 2 * (size_t)order;
+  const int last = r[2] > 1 ? r[2] : r[1];
   for (int k1 = 0; k1 < r[0]; ++k1)
     for (int k2 = 0; k2 < r[1]; ++k2)
       for (int k3 = 0; k3 < r[2]; ++k3) {
         const int f = k1 + r[0] * k2 + r[0] * r[1] * k3;
-        float* s = spec + 2 * (size_t)((k1 * r[1] + k2) * r[2] + k3);
+        const int pos = (k1 * r[1] + k2) * r[2] + k3;
+        float* s = spec + 2 * (size_t)(pos % last * (order / last) + pos / last);
         // 1 / (1 - exp(-i w)) = (1 - i cot(w / 2)) / 2
         s[0] = (float)(f ? H[f] / (2.0 * order) : H[0] / order);
         s[1] = (float)(f ? -H[f] / (2.0 * order * std::tan(pi * f / order)) : 0.0);
       }
-  for (int k = 0; k < order; ++k) {
-    tw[2 * k] = (float)ct[k];
-    tw[2 * k + 1] = (float)-std::sin(2.0 * pi * k / order);
+  for (int pass = 0; pass < (r[2] > 1 ? 2 : 1); ++pass) {
+    const int rows = pass ? r[2] : order / r[0], f = pass ? r[0] : 1;
+    for (int k = 0; k < 4; ++k)
+      for (int n = 0; n < rows; ++n) {
+        const int a = ((n * f) << k) % order;
+        *tw++ = (float)ct[a];
+        *tw++ = (float)-std::sin(2.0 * pi * a / order);
+      }
   }
 }
 
