@@ -2,7 +2,7 @@
 // MEXCT_FP_RAY and MEXCT_FP_TEXTURE variants), voxel-driven backprojectors
 // (standard BP, OSC dual BP + update, batched BP) and the general3D scatter
 // backprojector for sm_103a.  The standard and OSC forward projections run
-// in the slab kernel of k_slab.cu.
+// in k_slab.cu (cone) and k_rows.cu (parallel, fan).
 //
 // Ray-per-thread FP (CUDAmex_FP.cu:56-346, CUDAmex_general3D_FP.cu:59-150)
 //   One thread per detector pixel; a warp owns 32 consecutive pixels of one
@@ -485,28 +485,49 @@ __device__ __forceinline__ void bp_column_quad(const typename QuadT<S>::T* __res
 // packed operations per pair.  Row r = min(z, H - 1) with weight 1 (az = 0:
 // acc = fma(w0, P(r, iu), fma(w1, P(r, iu+1), acc))); the layout clamps row
 // r + 1 exactly as min(z + 1, H - 1) does.
-template <int GEOM, int ZC, typename S = float>
-__device__ __forceinline__ void bp_column_quadrows(const typename QuadT<S>::T* __restrict__ p,
-                                                   int W, int H, int Wp, int z0,
-                                                   const ColGeom<GEOM>& g, float* acc,
-                                                   int roff = 0) {
+struct RowTap {
+  uint32_t iu;
+  float w0, w1;
+};
+template <int GEOM>
+__device__ __forceinline__ RowTap row_tap(int W, const ColGeom<GEOM>& g) {
   const float cu = fminf(fmaxf(g.py, -4.0f), (float)W + 4.0f) - 0.5f;
   const float fu = floorf(cu);
   const float au = cu - fu;
   const int iu = min(max((int)fu, -kSinoPad), W) + kSinoPad;
-  const float w0 = g.w * (1.0f - au), w1 = g.w * au;
-  const typename QuadT<S>::T* col = p + iu;
+  return {(uint32_t)iu, g.w * (1.0f - au), g.w * au};
+}
+// next(): the tap of the following view, made beside this view's loads.  FIRST:
+// all loads before the first use; the parallel BP compiles to 66 registers with
+// it and 80 without (384^3 x 512: 6.3 and 11.1 ms), the fan BP to 80 registers
+// and a spill with it, 80 without (255^2 x 201 x 360: 1.53 and 1.48 ms).
+template <int ZC, typename S, bool FIRST, typename Next>
+__device__ __forceinline__ RowTap bp_column_quadrows(const typename QuadT<S>::T* __restrict__ p,
+                                                     int H, int Wp, int z0, const RowTap& g,
+                                                     float* acc, int roff, Next next) {
   static_assert(ZC % 2 == 0, "ZC must be even");
-  const float2 w02 = make_float2(w0, w0), w12 = make_float2(w1, w1);
+  const float2 w02 = make_float2(g.w0, g.w0), w12 = make_float2(g.w1, g.w1);
+  // the row is the same for the warp, the column a 32-bit offset into it
+  auto load = [&](int j) {
+    const typename QuadT<S>::T* row = p + (size_t)(min(z0 + j - roff, H - 1) + kSinoPad) * Wp;
+    return QuadT<S>::get(row + g.iu);
+  };
+  float4 q[ZC / 2];
+  if constexpr (FIRST) {
+#pragma unroll
+    for (int j = 0; j < ZC; j += 2) q[j / 2] = load(j);
+  }
+  const RowTap n = next();
 #pragma unroll
   for (int j = 0; j < ZC; j += 2) {
-    const float4 q = QuadT<S>::get(col + (size_t)(min(z0 + j - roff, H - 1) + kSinoPad) * Wp);
-    const float2 t = __ffma2_rn(w02, make_float2(q.x, q.y),
-                                __ffma2_rn(w12, make_float2(q.z, q.w),
+    const float4 c = FIRST ? q[j / 2] : load(j);
+    const float2 t = __ffma2_rn(w02, make_float2(c.x, c.y),
+                                __ffma2_rn(w12, make_float2(c.z, c.w),
                                            make_float2(acc[j], acc[j + 1])));
     acc[j] = t.x;
     acc[j + 1] = t.y;
   }
+  return n;
 }
 
 // Launch shape (BpShape): ZC z voxels per thread, blocks of 32 x rows
@@ -518,9 +539,12 @@ __device__ __forceinline__ void bp_column_quadrows(const typename QuadT<S>::T* _
 template <int GEOM, int ZC, typename TS, typename TV, int MODE = 0>
 // Cone columns take 16 bilinear taps per z pair; bounding registers to 64 keeps
 // 4 CTAs (32 warps) per SM resident, 5% faster at 512^3 x 720 than the 66
-// registers / 3 CTAs the compiler picks unbounded.  Par/fan columns need no
-// bound.
-__global__ void __launch_bounds__(256, GEOM == 2 ? 4 : 1) bp_pad_kernel(const __grid_constant__ VoxArgs A,
+// registers / 3 CTAs the compiler picks unbounded.  Par/fan columns wait on
+// their loads: 3 CTAs (80 registers) instead of the 2 of 88 to 95 registers took
+// 384^3 x 512 parallel from 8.1 to 6.3 ms, 255^2 x 201 x 360 fan from 1.80 to
+// 1.48 (4 CTAs: 6.3 and 1.96).  The decoupled detector's keep their z taps in
+// registers and take no bound.
+__global__ void __launch_bounds__(256, GEOM == 2 ? 4 : MODE == 1 ? 1 : 3) bp_pad_kernel(const __grid_constant__ VoxArgs A,
                                                      const TS* __restrict__ sino, int Wp,
                                                      TV* __restrict__ vol, int accumulate,
                                                      int nz, int vblocks,
@@ -573,14 +597,21 @@ __global__ void __launch_bounds__(256, GEOM == 2 ? 4 : 1) bp_pad_kernel(const __
       const int zg = MODE == 2 ? A.zoff + z0 : z0;
       const int roff = MODE == 2 ? A.row0 : 0;
       const size_t vstride = (size_t)Wp * (rows + 2 * kSinoPad);
-      for (int v = vbeg; v < vend; ++v) {
-        const ColGeom<GEOM> g = col_geom<GEOM>(x, y, A.trig[v], A.SR, A.v0, (float)A.hw, A.v0,
-                                               1.f, 1.f);
-        if constexpr (GEOM == 2)
+      if constexpr (GEOM == 2) {
+        for (int v = vbeg; v < vend; ++v) {
+          const ColGeom<GEOM> g = col_geom<GEOM>(x, y, A.trig[v], A.SR, A.v0, (float)A.hw, A.v0,
+                                                 1.f, 1.f);
           bp_column_quad<ZC, S>(q + (size_t)v * vstride, A.W, rows, Wp, zg, g, acc, roff);
-        else  // par / fan: the z rows are texel rows
-          bp_column_quadrows<GEOM, ZC, S>(q + (size_t)v * vstride, A.W, rows, Wp, zg, g, acc,
-                                          roff);
+        }
+      } else if (vbeg < vend) {  // par / fan: the z rows are texel rows
+        auto tap = [&](int v) {
+          return row_tap<GEOM>(A.W, col_geom<GEOM>(x, y, A.trig[v], A.SR, A.v0, (float)A.hw, A.v0,
+                                                   1.f, 1.f));
+        };
+        RowTap g = tap(vbeg);
+        for (int v = vbeg; v < vend; ++v)
+          g = bp_column_quadrows<ZC, S, GEOM == 0>(q + (size_t)v * vstride, rows, Wp, zg, g, acc, roff,
+                                        [&] { return tap(min(v + 1, vend - 1)); });
       }
     }
   }
@@ -1059,8 +1090,8 @@ cudaError_t launch_g3d_bp(const RayArgs& a, const float* sino,
 
 // ---------------------------------------------------------------------------
 // OSC kernels.  The subset FP with the residual epilogue
-// (CUDAmex_oscIter.cu:140-271) is the slab kernel of k_slab.cu with border
-// addressing and step 0.5.
+// (CUDAmex_oscIter.cu:140-271) is the slab kernel of k_slab.cu (cone) or the
+// rows kernel of k_rows.cu with border addressing and step 0.5.
 // ---------------------------------------------------------------------------
 // Dual BP of the residuals with border addressing (CUDAmex_oscIter.cu:305-356)
 // into register accumulators, then mu <- max(mu + mu*num/den, 0) inside the
@@ -1106,8 +1137,10 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
       bp_column_quad<ZC, SD>(qpre, A.W, A.H, Wp, z0, g, num);
       bp_column_quad<ZC, SD>(qpost, A.W, A.H, Wp, z0, g, den);
     } else {
-      bp_column_quadrows<GEOM, ZC, SD>(qpre, A.W, A.H, Wp, z0, g, num);
-      bp_column_quadrows<GEOM, ZC, SD>(qpost, A.W, A.H, Wp, z0, g, den);
+      const RowTap t = row_tap<GEOM>(A.W, g);
+      auto same = [&] { return t; };
+      bp_column_quadrows<ZC, SD, false>(qpre, A.H, Wp, z0, t, num, 0, same);
+      bp_column_quadrows<ZC, SD, false>(qpost, A.H, Wp, z0, t, den, 0, same);
     }
   }
   const size_t base = (size_t)iy * A.W + ix;
