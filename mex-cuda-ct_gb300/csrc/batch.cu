@@ -3,11 +3,12 @@
 //
 // A batch is planned once (padded-volume buffers, per-problem device
 // descriptors with TMA maps and trig tables); each operator then runs as a
-// fixed, capturable sequence: one batched padding launch plus one persistent
-// FP launch, or one sinogram-padding launch per problem plus one persistent BP
-// launch.  Persistent CTAs take work items
-// (problem, view, tile) / (problem, brick) from a global counter, so uneven
-// problems load-balance inside one launch.
+// fixed, capturable sequence.  FP: the cone problems by one batched padding
+// launch plus one persistent launch, whose CTAs take (problem, view, tile) items
+// from a global counter so that uneven problems balance inside it; beside it,
+// on forked streams, a layout launch and the rows kernel per parallel / fan
+// problem.  BP: a padding launch and the BP launches per problem, on forked
+// streams.
 #include <algorithm>
 #include <cstring>
 #include <memory>

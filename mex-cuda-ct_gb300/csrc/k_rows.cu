@@ -19,7 +19,7 @@
 //    warp owns four rays of each view and 128 rows: per column one 16-byte
 //    load of data per lane, one broadcast of the four weights, and 8 packed
 //    FMAs.
-//  - Calls of few views share a tile's planes in a cluster of four CTAs.
+//  - Calls of few views share a tile's planes in a cluster of four or eight CTAs.
 // What that moves: a column of shared memory is read once per 4 rays instead
 // of 4 taps per sample, and the weights cost ~200 instructions per ray and
 // plane for 128 rows.  Measured, slab kernel -> this: 384^3 x 512 parallel
@@ -590,8 +590,9 @@ long long rows_ctas(const RayArgs& a, int v) {
 // CTAs that share each tile's planes as a cluster: four for calls of few views,
 // whose CTAs would leave SMs idle (an OSC subset: 84^2 x 76, 25 views per
 // subset, an iteration of 5 subsets 568 us without, 350 with), eight where that
-// still leaves them idle (64^2 x 40, 3 views, 12 subsets: 366 -> 286 us).  The rule does not look at
-// the slices, so a slab of a volume is summed as the whole volume is.
+// still leaves them idle (64^2 x 40, 3 views, 12 subsets: 366 -> 286 us).  The
+// rule does not look at the slices, so a slab of a volume is summed as the whole
+// volume is.
 int rows_split(const RayArgs& a) {
   const long long n = (long long)std::max(a.nall, a.nviews) * ((a.det_w + kRU - 1) / kRU);
   return 8 * n <= device_sms() ? 8 : n <= device_sms() ? 4 : 1;

@@ -1,6 +1,7 @@
-// k_slab.cu -- slab-staged forward projection with TMA for the standard
-// geometries (CUDAmex_FP.cu:56-346) and the OSC forward pass
-// (CUDAmex_oscIter.cu:140-271).
+// k_slab.cu -- slab-staged forward projection with TMA: cone rays
+// (CUDAmex_FP.cu:56-346) with the OSC forward pass (CUDAmex_oscIter.cu:140-271),
+// general3D rays, and parallel / fan rays onto a decoupled detector whose rows
+// fall between slices.  Other parallel / fan rays stay in a slice: k_rows.cu.
 //
 // Why: a ray-per-thread march that fetches its 8 trilinear taps through L1
 // issues ~28 L1 wavefronts per warp-sample, because the 32 rays of a warp
@@ -14,14 +15,17 @@
 // a padded volume into shared memory ([z][a][f] with f fastest) and every
 // lane takes its samples whose a-tap lies in the slab from shared memory with
 // constant-offset loads.  Two buffers and two mbarriers overlap the copy of
-// slab j+1 with the sampling of slab j.  Shapes (measured on cone 512^3 x
-// 720): 4 taps per slab, boxes of 64 (f) x 5 (a) x <=20 (z) elements that
-// hold 99.9% of the bundles, copied as one 20-row box per slab (2-, 4-, 5-
-// and 10-row boxes for the rows the bundle needs were 1-5% slower: the
-// issuing thread stalls its warp), 4 CTAs of 256 threads per SM (<=64
-// registers, 50 KB of buffers each); 3 taps (4 or 5 CTAs/SM) and 2 taps
-// (5 CTAs/SM) were 12-32% slower.  Planning all slabs up front instead of one
-// slab ahead in warp 0 took 15% off the sweep.
+// slab j+1 with the sampling of slab j.  The box (SlabCfg) holds 99.9 % of the
+// bundles of cone 512^3 x 720 and is copied whole (2-, 4-, 5- and 10-row boxes
+// for the rows the bundle needs were 1-5 % slower: the issuing thread stalls
+// its warp), 4 CTAs of 256 threads per SM (<=64 registers, 57 KB of buffers
+// each); 3 taps (4 or 5 CTAs/SM) and 2 taps (5 CTAs/SM) were 12-32 % slower.
+// Planning all slabs up front instead of one slab ahead in warp 0 took 15 % off
+// the sweep.  The shared-memory loads bound it: 79 % of the data pipe's
+// wavefronts, 1.5 a load, from lanes in different a-planes; idle lanes cost no
+// wavefronts.  Counting each ray's samples per slab and repeating its last one
+// instead of a single-sample path raised the active lanes from 24.5 to 27.6
+// and ran 182.3 ms against 178.7.
 //
 // The padded volume has a one-voxel border (replicated edge for clamp
 // addressing, zeros for border addressing) and a fast-axis pitch rounded up
@@ -180,12 +184,11 @@ cudaError_t launch_pad_volume_sub(bool rows, const float* src, int W, int nz, bo
 constexpr int kSlabCtas = 4;                  // resident CTAs per SM (launch bounds)
 // Slab shape per projection geometry: F x A x Z boxes (f extent, a-planes =
 // taps + 1, z rows).  Cone rays spread in z along a slab, so cone slabs are 5
-// taps thick in 18-row boxes; par / fan rays keep their z (an 8-row tile spans
-// 8 rows), so their slabs are 8 taps thick in 12-row boxes: fewer slabs per
-// ray, less per-slab work.  Measured at 512^3 x 720: cone 187.0 -> 180.8 ms,
-// par 202.6 -> 173.9 ms against 4 taps in 20 rows for both.  One box fills a
-// buffer; the buffers are sized for the larger shape, so the batched kernel
-// has one shared-memory size for every geometry.
+// taps thick in 18-row boxes; par / fan rays (of a decoupled detector) keep
+// their z (an 8-row tile spans 8 rows), so their slabs are 8 taps thick in
+// 12-row boxes: fewer slabs per ray, less per-slab work.  Measured at 512^3 x
+// 720: cone 187.0 -> 180.8 ms, par 202.6 -> 173.9 ms against 4 taps in 20 rows
+// for both.  One box fills a buffer; the buffers are sized for the larger shape.
 constexpr int kConeF = 64, kConeT = 5, kConeZ = 18;
 constexpr int kParF = 64, kParT = 8, kParZ = 12;
 template <int GEOM>

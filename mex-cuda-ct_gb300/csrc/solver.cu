@@ -7,7 +7,7 @@
 // whole reconstruction; an iteration is a fixed sequence of kernels:
 //
 //   mu_old <- mu                                     (:45)
-//   per subset: pad(mu), slab FP + residual, dual BP + update         (:51-59)
+//   per subset: slab / rows FP + residual, dual BP + update           (:51-59)
 //   k > 1: d_a = ||mu_old - mu|| in FP64 (mu_old(1) = 0, NaN dropped)  (:64-67)
 //          20 TV steps with c = TV_constant * d_a read on the device    (:68)
 //          NaN/Inf -> 0                                                 (:69-70)
