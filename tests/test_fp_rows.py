@@ -86,3 +86,18 @@ def test_a_voxel_that_is_not_finite_reaches_its_own_rays_only(cuda, geom):
         assert np.isnan(got[int(round(u)), z, k])
     rest = np.arange(H) != z
     assert np.array_equal(got[:, rest], clean[:, rest])
+
+
+@pytest.mark.parametrize("geom", [0, 1])
+@pytest.mark.parametrize("Wd,du", [(75, 0.8), (90, 1.3), (20, 1.0), (33, 2.5)])
+def test_decoupled_columns(cuda, orc, geom, Wd, du):
+    """Detector rows that are the volume's slices, columns of their own: rays that miss
+    the volume, and tiles wider than the staged box."""
+    from mexct import ops
+
+    W, H = 48, 21
+    rng = np.random.default_rng(Wd)
+    vol = np.asfortranarray(rng.uniform(0, 1, (W, W, H)).astype(np.float32))
+    ang = np.deg2rad(10 + 29.0 * np.arange(11)).astype(np.float32)
+    got = _host(ops.fp_det_dev(_dev(vol), 300.0, ang, geom, Wd, H, du, 1.0, 1))
+    assert rel_l2(got, orc.fp_det(vol, 300.0, ang, geom, Wd, H, du, 1.0, 1)) <= 1e-5
