@@ -1117,7 +1117,7 @@ __global__ void __launch_bounds__(256) prefilter_tiled_kernel(
 // through shared memory for 3 radices.  The zero half of the padded row
 // (W <= N / 2) is never loaded, and only the first half is transformed back.
 // Rows move through memory once: 8 bytes per pixel.  384^2 x 512 views, cone,
-// Hamming: 2.47 -> 0.49 ms (1.24 TB/s: issue slots 70 % and the shared / L1 data
+// Hamming: 2.47 -> 0.50 ms (1.2 TB/s: issue slots 70 % and the shared / L1 data
 // path 61 %, not the memory, bound it); 3 CTAs of 80 registers per SM.  With so
 // few warps the order of the loads counts: tables laid out so that a warp reads
 // neighbours took it from 0.70 to 0.63 ms (the spectrum, 64 bytes apart, had
@@ -1130,6 +1130,13 @@ __global__ void __launch_bounds__(256) prefilter_tiled_kernel(
 // x[u-1] are transformed and the spectrum is divided by 1 - exp(-i w): what is
 // transformed is as small as the output.  The sum of a row, which differences
 // lose, is taken beside them and is the transform's element 0.
+//
+// The twiddle products mix the two rows of a pair, so rounding is relative to
+// the larger one: each row is scaled by the power of two that brings its largest
+// magnitude into [1, 2) and back at the store (exact, so a pair of like rows
+// gives the bits that it gives unscaled; without it a row beside one 1e4 times
+// larger was off by 4e-4; 15 us of 502 at 384^2 x 512).  A row of zeros stores
+// zeros.
 //
 // A row with a value that is not finite or above 1e30 would reach its partner
 // (and could overflow in a sum the direct form does not take): such rows enter
@@ -1251,6 +1258,18 @@ __device__ __forceinline__ float prefilter_fast_input(const FiltArgs& A, float s
   return s * pk;
 }
 
+// 2^-e and 2^e of a row's largest magnitude m = 2^e (1 .. 2), e >= -126; for a
+// row of zeros 2^e is 0.
+__device__ __forceinline__ unsigned row_exp(float m) {
+  return min(max(__float_as_uint(m) >> 23, 1u), 253u);
+}
+__device__ __forceinline__ float row_scale(float m) {
+  return __uint_as_float((254u - row_exp(m)) << 23);
+}
+__device__ __forceinline__ float row_unscale(float m) {
+  return m > 0.f ? __uint_as_float(row_exp(m) << 23) : 0.f;
+}
+
 constexpr int kFftThreads = 256, kFftElems = 16 * kFftThreads;  // complex elements per CTA
 
 template <int R1, int R2, int R3>
@@ -1263,7 +1282,7 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   __shared__ float2 sm[kFftElems + kFftElems / 8];
   __shared__ int bad[2 * NF];  // rows kept out of the transform
   constexpr int TW = TF < 32 ? TF : 32, NWF = TF / TW;  // lanes and warps per transform
-  __shared__ float2 psum[NF * NWF], edge[8 * NF * NWF];
+  __shared__ float2 psum[NF * NWF], pmax[NF * NWF], edge[8 * NF * NWF];
   // after the spatial kernel: the differences' spectrum and the twiddles
   const float2* spec = reinterpret_cast<const float2*>(kern + N);
   const float2 *tw1 = spec + N, *tw2 = tw1 + 4 * TF;
@@ -1315,29 +1334,49 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
     if (b0) bad[2 * q] = 1;
     if (b1) bad[2 * q + 1] = 1;
   }
-  // row sums, and each element's left neighbour: lane n - 1, whose warp leaves
-  // its last lane's elements in edge
+  // row sums and largest magnitudes, and each element's left neighbour: lane n -
+  // 1, whose warp leaves its last lane's elements in edge
   const int wq = q * NWF + n / TW;
-  float2 sum = make_float2(0.f, 0.f), left[8];
+  float2 sum = make_float2(0.f, 0.f), big = sum, left[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) sum = c_add(sum, e[j]);
+  for (int j = 0; j < 8; ++j) {
+    sum = c_add(sum, e[j]);
+    big = make_float2(fmaxf(big.x, fabsf(e[j].x)), fmaxf(big.y, fabsf(e[j].y)));
+  }
 #pragma unroll
   for (int o = TW / 2; o > 0; o >>= 1) {
     sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
     sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+    big.x = fmaxf(big.x, __shfl_xor_sync(0xffffffffu, big.x, o));
+    big.y = fmaxf(big.y, __shfl_xor_sync(0xffffffffu, big.y, o));
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     left[j].x = __shfl_up_sync(0xffffffffu, e[j].x, 1, TW);
     left[j].y = __shfl_up_sync(0xffffffffu, e[j].y, 1, TW);
   }
-  if (n % TW == 0) psum[wq] = sum;
+  if (n % TW == 0) {
+    psum[wq] = sum;
+    pmax[wq] = big;
+  }
   if (n % TW == TW - 1) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) edge[8 * wq + j] = e[j];
   }
   const bool any = __syncthreads_or(b0 || b1) != 0;
   const bool bad0 = bad[2 * q] != 0, bad1 = bad[2 * q + 1] != 0;
+  // 2^-e of both rows, or 2^e (back); read again at the store instead of kept
+  auto scales = [&](bool back) {
+    float2 m = pmax[q * NWF];
+#pragma unroll
+    for (int w = 1; w < NWF; ++w) {
+      const float2 b = pmax[q * NWF + w];
+      m = make_float2(fmaxf(m.x, b.x), fmaxf(m.y, b.y));
+    }
+    return back ? make_float2(row_unscale(m.x), row_unscale(m.y))
+                : make_float2(row_scale(m.x), row_scale(m.y));
+  };
+  const float2 scale = scales(false);
   float2 past = make_float2(0.f, 0.f);  // element N / 2 of the differences (thread 0)
   if (n % TW == 0) {
     const float2* ed = edge + 8 * (n == 0 ? q * NWF + NWF - 1 : wq - 1);
@@ -1347,8 +1386,8 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
     if (n == 0) past = make_float2(-ed[7].x, -ed[7].y);
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) e[j] = c_sub(e[j], left[j]);
-  e[8] = past;
+  for (int j = 0; j < 8; ++j) e[j] = __fmul2_rn(c_sub(e[j], left[j]), scale);
+  e[8] = __fmul2_rn(past, scale);
   if (any) {
 #pragma unroll
     for (int j = 0; j <= 8; ++j) {
@@ -1395,6 +1434,7 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
         e[0] = psum[q * NWF];
 #pragma unroll
         for (int w = 1; w < NWF; ++w) e[0] = c_add(e[0], psum[q * NWF + w]);
+        e[0] = __fmul2_rn(e[0], scales(false));
         if (bad0) e[0].x = 0.f;
         if (bad1) e[0].y = 0.f;
       }
@@ -1427,12 +1467,13 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   twiddle<R1, true>(e, w1);
   dft<R1, true>(e);
   const float db = live ? __ldg(dbeta + view) : 0.f;
+  const float2 unscale = scales(true);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int u = n + j * TF;
     if (live && u < W) {
-      if (!bad0) out[row0 + u] = e[j].x * db;
-      if (two && !bad1) out[row0 + W + u] = e[j].y * db;
+      if (!bad0) out[row0 + u] = e[j].x * unscale.x * db;
+      if (two && !bad1) out[row0 + W + u] = e[j].y * unscale.y * db;
     }
   }
   if (any) {  // rows kept out: the direct sum, from staged inputs (out may be sino)
