@@ -47,7 +47,7 @@ SOURCES = [
 
 
 def available() -> bool:
-    return os.path.isdir(REF)
+    return all(os.path.isfile(os.path.join(REF, src)) for src, _, _ in SOURCES)
 
 
 def _nvcc() -> str:
