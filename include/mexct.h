@@ -427,6 +427,15 @@ mexct_status mexct_autotune_bp(mexct_ctx* ctx, const void* d_sino,
                                int vol_type, void* stream, mexct_shape* best,
                                double* best_ms);
 
+/* Which kernel a parallel / fan FP (nsub = 0) or the subsets of an OSC
+ * iteration (nsub >= 1: views i, i + nsub, ...) of a W x W x H volume run on, on
+ * a device of `sms` SMs (0: the current device): *rows = 1 the kernel that takes
+ * 128 slices at once (*views per CTA, clusters of *split CTAs), 0 the slab kernel
+ * (always for cone, and for volumes of few slices).  Host-only when sms > 0. */
+mexct_status mexct_fp_plan(int W, int H, float sad, const float* angles, int nP,
+                           int geom, int nsub, int sms, int* rows, int* views,
+                           int* split);
+
 /* ---- allocation-free variant ------------------------------------------ */
 
 /* TV descent for callers that cannot allocate device memory while they run.

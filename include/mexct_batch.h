@@ -28,8 +28,9 @@ typedef struct mexct_batch mexct_batch;
 mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int n,
                                 mexct_batch** out);
 /* FP of every problem: one batched padding launch + one persistent launch for
- * the cone problems, a layout launch and a launch of the rows kernel for each
- * parallel / fan problem, on streams forked from `stream` and joined back.
+ * the slab kernel's problems (cone; parallel / fan that are small or of few
+ * slices, see mexct_fp_plan), a layout launch and a launch of the rows kernel for
+ * each of the others, on streams forked from `stream` and joined back.
  * Stream-ordered, no host work, capturable in a CUDA graph. */
 mexct_status mexct_batch_fp(mexct_batch* b, void* stream);
 /* BP of every problem (d_sino -> d_rec): per problem a padding launch and its

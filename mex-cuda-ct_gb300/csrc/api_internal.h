@@ -151,10 +151,12 @@ struct DevGuard {
 
 inline size_t dsize(int t) { return t == kF32 ? 4 : 2; }
 
-// rows: the z-fastest layout (fp_uses_rows geometries), else the slab kernel's.
+// rows: the z-fastest layout (fp_uses_rows), else the slab kernel's.
 mexct_status prepare_slab_bufs(Buf& px, Buf& py, Buf& err, const void* d_vol, int vt, int W,
                                int H, bool border, int geom, bool rows, CUtensorMap* mx,
                                CUtensorMap* my, int* Pf_out, cudaStream_t st);
+bool subset_uses_rows(int geom, int W, int H, int nz, float sad, const float* angles, int nP,
+                      int nsub, int epi);
 mexct_status osc_tv_recon_typed(mexct_ctx* ctx, const float* pre, const float* post, int W, int H,
                                 int nP, const float* angles, float sad, int geom, int n_iter,
                                 float tv_const, int n_sub_init, int n_sub_final, float p_val,

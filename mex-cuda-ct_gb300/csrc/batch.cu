@@ -3,11 +3,11 @@
 //
 // A batch is planned once (padded-volume buffers, per-problem device
 // descriptors with TMA maps and trig tables); each operator then runs as a
-// fixed, capturable sequence.  FP: the cone problems by one batched padding
-// launch plus one persistent launch, whose CTAs take (problem, view, tile) items
-// from a global counter so that uneven problems balance inside it; beside it,
-// on forked streams, a layout launch and the rows kernel per parallel / fan
-// problem.  BP: a padding launch and the BP launches per problem, on forked
+// fixed, capturable sequence.  FP: the slab kernel's problems (fp_uses_rows) by
+// one batched padding launch plus one persistent launch, whose CTAs take (problem,
+// view, tile) items from a global counter so that uneven problems balance inside
+// it; beside it, on forked streams, a layout launch and the rows kernel per problem
+// of the others.  BP: a padding launch and the BP launches per problem, on forked
 // streams.
 #include <algorithm>
 #include <cstring>
@@ -29,7 +29,7 @@ struct mexct_batch {
   std::vector<mexct_problem> probs;
   // BP launch arguments per problem and view chunk (at most kMaxViews views)
   std::vector<std::vector<std::unique_ptr<VoxArgs>>> vox;
-  // parallel / fan FP: launch arguments per problem and view chunk, tensor maps
+  // FP problems on the rows kernel: launch arguments per view chunk, tensor maps
   std::vector<std::vector<std::unique_ptr<RayArgs>>> rays;
   std::vector<CUtensorMap> rmx, rmy;
   Buf fp_desc, trig, counters, err;
@@ -100,7 +100,12 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
   for (int i = 0; i < n; ++i) {
     const mexct_problem& p = probs[i];
     const int W = p.W, H = p.H;
-    const bool rows = fp_uses_rows(p.geom);
+    std::unique_ptr<RayArgs> first(new RayArgs);
+    fill_std_rays(*first, W, H, p.sad, p.geom, false);
+    first->nall = p.nP;
+    first->nviews = std::min(kMaxViews, p.nP);
+    for (int v = 0; v < first->nviews; ++v) trig_of(p.angles[v], &first->trig[v]);
+    const bool rows = fp_uses_rows(p.geom, *first, H, 0);  // as mexct_fp_dev
     const FpLayout L = fp_layout(rows, W, H, kF32);
     const int Pf = L.pitch;
     MEXCT_TRY_CUDA(b->pads[2 * i].ensure(L.px), "batch_create: padded volume");
@@ -116,13 +121,12 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
       b->rmy[i] = f.tmy;
       const SlabEpi none{nullptr, nullptr, nullptr, nullptr, nullptr};
       for (int v0 = 0; v0 < p.nP; v0 += kMaxViews) {
-        std::unique_ptr<RayArgs> ra(new RayArgs);
-        fill_std_rays(*ra, W, H, p.sad, p.geom, false);
+        std::unique_ptr<RayArgs> ra(new RayArgs(*first));
+        ra->nviews = 0;
         if (v0 == 0)  // kernel attributes, before any capture
           MEXCT_TRY_CUDA(launch_fp_rows(p.geom, 0, *ra, f.tmx, f.tmy, b->pads[2 * i].p, Pf, kF32,
                                         nullptr, kF32, none, nullptr),
                          "batch_create: kernel setup");
-        ra->nall = p.nP;
         ra->nviews = std::min(kMaxViews, p.nP - v0);
         ra->view0 = v0;
         for (int v = 0; v < ra->nviews; ++v) trig_of(p.angles[v0 + v], &ra->trig[v]);
@@ -143,7 +147,7 @@ mexct_status mexct_batch_create(mexct_ctx* ctx, const mexct_problem* probs, int 
     f.sad = p.sad;
     f.step = p.geom == 2 ? 1.0f : 0.5f;
     f.item0 = b->fp_items;
-    // parallel / fan problems have launches of their own: no items here
+    // the rows kernel's problems have launches of their own: no items here
     if (!rows) b->fp_items += (long long)p.nP * f.tiles_u * ((H + 7) / 8);
     f.px = b->pads[2 * i].p;
     f.py = b->pads[2 * i + 1].p;
@@ -184,8 +188,8 @@ mexct_status mexct_batch_fp(mexct_batch* b, void* stream) {
   DevGuard dg(b->device);
   NvtxRange nvtx("mexct:batch_fp");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // parallel / fan problems beside the persistent launch of the cone problems,
-  // on the streams the BP uses
+  // the rows kernel's problems beside the persistent launch of the others, on the
+  // streams the BP uses
   MEXCT_TRY_CUDA(cudaEventRecord(b->fork, st), "batch_fp: fork");
   bool used[mexct_batch::kAux] = {};
   for (int i = 0, k = 0; i < b->n; ++i) {

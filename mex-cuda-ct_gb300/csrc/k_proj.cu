@@ -1099,7 +1099,9 @@ cudaError_t launch_g3d_bp(const RayArgs& a, const float* sino,
 // DET: a decoupled detector (A.det_w x A.det_h pixels of reciprocal pitch
 // A.inv_du, A.inv_dv; no counterpart in the reference): every geometry
 // interpolates its residuals in v, as the detector BP does.
-template <int GEOM, int ZC, typename TM, bool DET = false, typename SD = float>
+// ROWS: the padded copy of mu is the rows FP's (a template: with both layouts in
+// one kernel the parallel form took 43 registers instead of 35).
+template <int GEOM, int ZC, typename TM, bool DET = false, typename SD = float, bool ROWS = false>
 __global__ void __launch_bounds__(256) osc_bp_update_kernel(
     const __grid_constant__ VoxArgs A, const void* __restrict__ rpre,
     const void* __restrict__ rpost, TM* __restrict__ mu, TM* __restrict__ padx,
@@ -1146,11 +1148,11 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
   const size_t base = (size_t)iy * A.W + ix;
   const size_t sz = (size_t)A.W * A.W;
   const size_t Ps = (size_t)A.W + 2;
-  // parallel / fan: the FP's z-fastest layout (columns of pitch Pf, a multiple
-  // of four as zl is): a column's FP32 slices in one store
-  constexpr bool rows = GEOM < 2 && !DET;
-  TM* const col = rows && padx ? padx + ((size_t)(iy + 1) * Ps + (ix + 1)) * Pf + zl : nullptr;
-  const bool whole = rows && std::is_same<TM, float>::value && ZC == 4 && zl + ZC <= A.nzs;
+  // the rows FP's z-fastest layout (columns of pitch Pf, a multiple of four as zl
+  // is): a column's FP32 slices in one store
+  static_assert(!ROWS || (GEOM < 2 && !DET), "rays that stay in a slice");
+  TM* const col = ROWS ? padx + ((size_t)(iy + 1) * Ps + (ix + 1)) * Pf + zl : nullptr;
+  const bool whole = ROWS && std::is_same<TM, float>::value && ZC == 4 && zl + ZC <= A.nzs;
   float4 four = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int j = 0; j < ZC; ++j) {
@@ -1160,9 +1162,9 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
       const float f = ldp(o);
       const float m = fmaxf(f + (f * num[j] / den[j]), 0.f);
       stf(o, m);
-      if (rows) {
+      if (ROWS) {
         if (whole) (&four.x)[j & 3] = m;
-        else if (col) stf(col + j, m);
+        else stf(col + j, m);
       } else if (padx) {
         // the slab FP's padded layouts: x-fastest and y-fastest, frame of one
         const size_t zp = (size_t)(z + 1) * Ps;
@@ -1171,7 +1173,7 @@ __global__ void __launch_bounds__(256) osc_bp_update_kernel(
       }
     }
   }
-  if (rows && whole && col) *reinterpret_cast<float4*>(col) = four;
+  if (ROWS && whole) *reinterpret_cast<float4*>(col) = four;
 }
 
 cudaError_t launch_osc_bp_update_det(int geom, const VoxArgs& a, const float* rpre,
@@ -1198,33 +1200,29 @@ cudaError_t launch_osc_bp_update(int geom, const VoxArgs& a,
   if (a.zoff % ZC != 0 || a.zoff < 0 || a.nzs < 1 || a.zoff + a.nzs > a.H)
     return cudaErrorInvalidValue;
   dim3 blk(32, 8), grd((a.W + 31) / 32, (a.W + 7) / 8, (a.nzs + ZC - 1) / ZC);
+#define OSC_BP(G, T, SD, R)                                                              \
+  osc_bp_update_kernel<G, ZC, T, false, SD, R><<<grd, blk, 0, st>>>(a, rpre, rpost, (T*)mu, \
+                                                                    (T*)padx, (T*)pady, Pf)
+#define OSC_GO(T, SD)                                   \
+  do {                                                  \
+    if (geom == 2) OSC_BP(2, T, SD, false);             \
+    else if (geom == 0 && rows) OSC_BP(0, T, SD, true); \
+    else if (geom == 0) OSC_BP(0, T, SD, false);        \
+    else if (rows) OSC_BP(1, T, SD, true);              \
+    else OSC_BP(1, T, SD, false);                       \
+  } while (0)
+  const bool rows = geom != 2 && !pady;
   if (dt == kF16) {  // FP16 residual views (FP32 mu)
     if (mt != kF32) return cudaErrorInvalidValue;
-#define OSC_BP16(G)                                                                      \
-  osc_bp_update_kernel<G, ZC, float, false, __half><<<grd, blk, 0, st>>>(                \
-      a, rpre, rpost, (float*)mu, (float*)padx, (float*)pady, Pf)
-    if (geom == 0) OSC_BP16(0);
-    else if (geom == 1) OSC_BP16(1);
-    else OSC_BP16(2);
-#undef OSC_BP16
-    return cudaGetLastError();
-  }
-#define OSC_BP(G, T)                                                                 \
-  osc_bp_update_kernel<G, ZC, T><<<grd, blk, 0, st>>>(a, rpre, rpost, (T*)mu, (T*)padx, \
-                                                      (T*)pady, Pf)
-  if (mt == kF32) {
-    if (geom == 0) OSC_BP(0, float);
-    else if (geom == 1) OSC_BP(1, float);
-    else OSC_BP(2, float);
+    OSC_GO(float, __half);
+  } else if (mt == kF32) {
+    OSC_GO(float, float);
   } else if (mt == kF16) {
-    if (geom == 0) OSC_BP(0, __half);
-    else if (geom == 1) OSC_BP(1, __half);
-    else OSC_BP(2, __half);
+    OSC_GO(__half, float);
   } else {
-    if (geom == 0) OSC_BP(0, __nv_bfloat16);
-    else if (geom == 1) OSC_BP(1, __nv_bfloat16);
-    else OSC_BP(2, __nv_bfloat16);
+    OSC_GO(__nv_bfloat16, float);
   }
+#undef OSC_GO
 #undef OSC_BP
   return cudaGetLastError();
 }

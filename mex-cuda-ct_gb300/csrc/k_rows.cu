@@ -593,16 +593,16 @@ long long rows_ctas(const RayArgs& a, int v) {
 // still leaves them idle (64^2 x 40, 3 views, 12 subsets: 366 -> 286 us).  The
 // rule does not look at the slices, so a slab of a volume is summed as the whole
 // volume is.
-int rows_split(const RayArgs& a) {
+int rows_split(const RayArgs& a, int sms) {
   const long long n = (long long)std::max(a.nall, a.nviews) * ((a.det_w + kRU - 1) / kRU);
-  return 8 * n <= device_sms() ? 8 : n <= device_sms() ? 4 : 1;
+  return 8 * n <= sms ? 8 : n <= sms ? 4 : 1;
 }
 
 // Views per CTA: four or two where the CTAs still fill the GPU and their
 // rays' columns of one plane fit the box (neighbouring rays at 45 degrees are
 // up to sqrt(2) times the magnification apart; a view shifts by its angle times
 // the half diagonal; what does not fit is read from global memory), else one.
-int rows_views(int geom, const RayArgs& a) {
+int rows_views(int geom, const RayArgs& a, int sms) {
   const double R = 0.7072 * a.S;
   const double mag = geom == 1 ? std::min(1.0 + R / std::max((double)a.SR, 1.0), 2.0) : 1.0;
   const double tile = std::min(kRU, a.det_w) * 1.4143 * mag * a.du;
@@ -613,7 +613,7 @@ int rows_views(int geom, const RayArgs& a) {
   }
   const double worst = std::acos(std::max(-1.0, cmin));
   for (int v : {4, 2})
-    if (rows_ctas(a, v) >= 2ll * device_sms() && tile + (v - 1) * worst * R + 4.0 <= kRF + 2.0)
+    if (rows_ctas(a, v) >= 2ll * sms && tile + (v - 1) * worst * R + 4.0 <= kRF + 2.0)
       return v;
   return 1;
 }
@@ -674,16 +674,51 @@ cudaError_t rows_launch(int geom, const RayArgs& a, const CUtensorMap& mx, const
   }
   // (the objective's partials have room for one CTA per tile)
   if constexpr (EPI != 2) {
-    const int sp = rows_split(a);
+    const int sp = rows_split(a, device_sms());
     if (sp == 8) return GO(1, 4, 8, false);
     if (sp == 4) return 4 * rows_ctas(a, 1) > device_sms() ? GO(1, 2, 4, false) : GO(1, 4, 4, false);
   }
-  const int v = rows_views(geom, a);
+  const int v = rows_views(geom, a, device_sms());
   return v == 4 ? GO(4, 2, 1, false) : v == 2 ? GO(2, 2, 1, false) : GO(1, 2, 1, false);
 #undef GO
 }
 
 }  // namespace
+
+void fp_rows_shape(int geom, const RayArgs& a, int epi, int sms, int* views, int* split) {
+  *split = epi == 2 ? 1 : rows_split(a, sms);
+  *views = *split > 1 ? 1 : rows_views(geom, a, sms);
+}
+
+// A CTA of the rows kernel works on 128 slices whatever nz is; the slab kernel's
+// work goes with its tiles of eight rows.  A plane of the sweep takes a slab CTA
+// (four per SM) 0.29 us and a rows CTA (two per SM) of 1 / 2 / 4 views 0.80 / 1.33
+// / 2.3 us, so a wave of the rows kernel costs as much as 2.75 / 4.6 / 7.9 waves of
+// the slab kernel (a part-filled last wave counted half full).  Measured, slab ->
+// rows at 16, 32, 48, 64 slices: 512^2 x 720 parallel 5.5 -> 11.0, 10.8 -> 11.0,
+// 16.1 -> 11.1, 21.4 -> 11.1 ms (one slice: 1.5 -> 11.0); 128^2 x 180 156 -> 326,
+// 248 -> 328, 348 -> 330, 447 -> 324 us; 512^2 x 90 0.77 -> 1.98, 1.47 -> 1.98, 2.18
+// -> 1.99, 2.88 -> 1.99 ms.
+// Clusters (few views) fill idle SMs: an OSC subset of 6 views of 256^2 breaks even
+// at eight slices, one of 5 views of 64^2 gains at one.  Line integrals also run in
+// batches, whose problems must agree with single calls bit for bit: there other
+// problems fill the SMs, the clusters pay from 49 slices on, and each rows problem
+// is two launches, which a problem of less than ~10 us of the slab kernel does not
+// make up for (64 problems 32^3 x 30: slab 228, rows 603 us).
+bool fp_uses_rows(int geom, const RayArgs& a, int nz, int epi, int sms) {
+  if ((geom != 0 && geom != 1) || a.nviews <= 0) return false;
+  if (sms <= 0) sms = device_sms();
+  const long long views = std::max(a.nall, a.nviews), tiles_u = (a.det_w + kRU - 1) / kRU;
+  const long long bundles = views * tiles_u, tz = (nz + 7) / 8;
+  if (epi == 0 && bundles * tz * (a.S + 2) < 12000) return false;
+  int v, split;
+  fp_rows_shape(geom, a, epi, sms, &v, &split);
+  if (split > 1) return epi == 0 ? tz > 6 : tz > 1 || 4 * bundles <= sms;
+  const double wave = (double)((views + v - 1) / v * tiles_u) / (2.0 * sms);
+  const double rows = std::max(1.0, 0.5 * (wave + std::ceil(wave)));
+  const double slab = (double)(bundles * tz) / (4.0 * sms);
+  return slab > rows * (v == 4 ? 7.9 : v == 2 ? 4.6 : 2.75);
+}
 
 int rows_pitch(int nz, int dtype) {
   const int unit = dtype == kF32 ? 4 : 8;  // 16-byte rows for TMA

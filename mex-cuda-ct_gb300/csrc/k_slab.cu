@@ -1070,7 +1070,9 @@ __global__ void __launch_bounds__(256, kSlabCtas) fp_batch_kernel(
     J.tu0 = (tile % B.tiles_u) * 32;
     J.tv0 = (tile / B.tiles_u) * 8;
     J.tmx = &B.tmx; J.tmy = &B.tmy; J.px = B.px; J.py = B.py; J.out = B.out;
-    slab_tile<2, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
+    if (B.geom == 0) slab_tile<0, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
+    else if (B.geom == 1) slab_tile<1, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
+    else slab_tile<2, 0, TV, TV>(J, buf0, buf1, S, phase, issued, E);
   }
 }
 
@@ -1246,7 +1248,7 @@ cudaError_t launch_fp_slab_g3d(const RayArgs& a, const CUtensorMap& mx, const CU
 cudaError_t launch_fp_slab_sub(int geom, const RayArgs& a, const CUtensorMap& mx,
                                const CUtensorMap& my, const void* px, const void* py, int Pf,
                                float* out, const SlabEpi& e, cudaStream_t st) {
-  if (fp_uses_rows(geom)) {
+  if (!py) {
     // a slab's rays reach its own rows only: the others' integrals are zero
     const int lo = a.zoff, hi = a.zoff + a.zrows - 2;  // rows lo .. hi - 1
     for (int part = 0; part < 2 && !a.accum && a.nviews > 0; ++part) {
@@ -1259,6 +1261,10 @@ cudaError_t launch_fp_slab_sub(int geom, const RayArgs& a, const CUtensorMap& mx
     }
     return launch_fp_rows(geom, 0, a, mx, my, px, Pf, kF32, out, kF32, e, st);
   }
+  if (geom == 0)
+    return slab_go<0, false, 0, float, float, false, true>(a, mx, my, px, py, Pf, out, e, st);
+  if (geom == 1)
+    return slab_go<1, false, 0, float, float, false, true>(a, mx, my, px, py, Pf, out, e, st);
   if (geom == 2)
     return slab_go<2, false, 0, float, float, false, true>(a, mx, my, px, py, Pf, out, e, st);
   return cudaErrorInvalidValue;
@@ -1268,9 +1274,11 @@ cudaError_t launch_fp_slab_objective(int geom, const RayArgs& a, const CUtensorM
                                      const CUtensorMap& my, const void* px, const void* py,
                                      int Pf, int vt, const SlabEpi& e, cudaStream_t st) {
   if (!e.obj || !e.pre || !e.post) return cudaErrorInvalidValue;
-  if (fp_uses_rows(geom))
-    return launch_fp_rows(geom, 2, a, mx, my, px, Pf, vt, nullptr, kF32, e, st);
-#define GO(TV) return slab_go<2, true, 2, TV, float>(a, mx, my, px, py, Pf, nullptr, e, st)
+  if (!py) return launch_fp_rows(geom, 2, a, mx, my, px, Pf, vt, nullptr, kF32, e, st);
+#define GO(TV)                                                                                 \
+  return geom == 0   ? slab_go<0, true, 2, TV, float>(a, mx, my, px, py, Pf, nullptr, e, st)   \
+         : geom == 1 ? slab_go<1, true, 2, TV, float>(a, mx, my, px, py, Pf, nullptr, e, st)   \
+                     : slab_go<2, true, 2, TV, float>(a, mx, my, px, py, Pf, nullptr, e, st)
   if (vt == kF32) GO(float);
   if (vt == kF16) GO(__half);
   GO(__nv_bfloat16);
@@ -1282,9 +1290,11 @@ cudaError_t launch_fp_slab(int geom, bool border, bool osc, const RayArgs& a,
                            const void* py, int Pf, int vt, void* out, int ot,
                            const SlabEpi& e, cudaStream_t st) {
   (void)border;
-  if (fp_uses_rows(geom))
-    return launch_fp_rows(geom, osc ? 1 : 0, a, mx, my, px, Pf, vt, out, ot, e, st);
-#define GO(B, EP, TV, TO) return slab_go<2, B, EP, TV, TO>(a, mx, my, px, py, Pf, out, e, st)
+  if (!py) return launch_fp_rows(geom, osc ? 1 : 0, a, mx, my, px, Pf, vt, out, ot, e, st);
+#define GO(B, EP, TV, TO)                                                                   \
+  return geom == 0   ? slab_go<0, B, EP, TV, TO>(a, mx, my, px, py, Pf, out, e, st)         \
+         : geom == 1 ? slab_go<1, B, EP, TV, TO>(a, mx, my, px, py, Pf, out, e, st)         \
+                     : slab_go<2, B, EP, TV, TO>(a, mx, my, px, py, Pf, out, e, st)
   if (osc) {
     // ot: storage of the residual views (FP16 with FP32 mu only)
     if (ot == kF16) {

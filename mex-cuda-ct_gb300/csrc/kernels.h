@@ -135,6 +135,8 @@ cudaError_t launch_sum_partials(const double* partials, long long n, double* out
 cudaError_t launch_combine_norms(const double* parts, int n, double* out, float c,
                                  const double* cmul, float* scale, cudaStream_t st);
 
+// px, py: the slab layouts, or the z-fastest one and null (the rows kernel), in
+// this and the other launches that take them.
 cudaError_t launch_fp_slab(int geom, bool border, bool osc, const RayArgs& a,
                            const CUtensorMap& mx, const CUtensorMap& my,
                            const void* px, const void* py, int Pf, int vt,
@@ -189,10 +191,15 @@ cudaError_t launch_fp_rows(int geom, int epi, const RayArgs& a, const CUtensorMa
                            const CUtensorMap& my, const void* vol, int Ph, int vt, void* out,
                            int ot, const SlabEpi& e, cudaStream_t st);
 
-// The volume layouts that the FP of a geometry reads.  Rays that stay in a
-// slice (parallel, fan) read one z-fastest copy (rows: px, and py is unused);
-// cone and general3D rays read the x-fastest and y-fastest copies.
-inline bool fp_uses_rows(int geom) { return geom == 0 || geom == 1; }
+// The volume layouts that an FP reads.  The rows kernel (rays that stay in a
+// slice: parallel, fan) reads one z-fastest copy (rows: px; py is null in the
+// launches below); the slab kernel reads the x-fastest and y-fastest copies.
+// fp_uses_rows: which of them serves the FP of nz slices with the rays of a
+// (its first launch's views, nall in all) and epilogue epi (launch_fp_rows), on
+// a device of `sms` SMs (0: the current one).  fp_rows_shape: views per CTA and
+// CTAs per cluster of the rows kernel's launch.
+bool fp_uses_rows(int geom, const RayArgs& a, int nz, int epi, int sms = 0);
+void fp_rows_shape(int geom, const RayArgs& a, int epi, int sms, int* views, int* split);
 struct FpLayout {
   size_t px, py;  // bytes
   int pitch;      // the launches' Pf

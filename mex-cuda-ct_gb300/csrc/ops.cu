@@ -111,6 +111,20 @@ mexct_status prepare_slab_bufs(Buf& px, Buf& py, Buf& err, const void* d_vol, in
   return MEXCT_OK;
 }
 
+// fp_uses_rows of the subsets of an OSC iteration (views i, i + nsub, ...; the
+// largest decides for all, for they share mu's layout), or of the objective.
+bool subset_uses_rows(int geom, int W, int H, int nz, float sad, const float* angles, int nP,
+                      int nsub, int epi) {
+  if (geom == 2 || nP <= 0) return false;
+  std::unique_ptr<RayArgs> a(new RayArgs);
+  fill_std_rays(*a, W, H, sad, geom, /*osc=*/true);
+  a->zrows = nz + 2;
+  a->nall = (nP + nsub - 1) / nsub;
+  a->nviews = std::min(kMaxViews, a->nall);
+  for (int i = 0; i < a->nviews; ++i) trig_of(angles[(size_t)i * nsub], &a->trig[i]);
+  return fp_uses_rows(geom, *a, nz, epi);
+}
+
 mexct_status prepare_slab(mexct_ctx* c, const void* d_vol, int vt, int W, int H,
                           bool border, int geom, bool rows, CUtensorMap* mx, CUtensorMap* my,
                           int* Pf_out, cudaStream_t st) {
@@ -159,9 +173,12 @@ mexct_status fp_run(mexct_ctx* c, const void* d_vol, int vt, int W, int H, float
   if (variant == MEXCT_FP_EXPLICIT) {
     CUtensorMap mx, my;
     int Pf = 0;
-    mexct_status s = prepare_slab(c, d_vol, vt, W, H, false, geom, fp_uses_rows(geom), &mx, &my,
-                                  &Pf, st);
+    a->nviews = std::min(kMaxViews, nP);
+    for (int i = 0; i < a->nviews; ++i) trig_of(angles[i], &a->trig[i]);
+    const bool rows = fp_uses_rows(geom, *a, H, 0);
+    mexct_status s = prepare_slab(c, d_vol, vt, W, H, false, geom, rows, &mx, &my, &Pf, st);
     if (s) return s;
+    const void* py = rows ? nullptr : c->pady.p;
     SlabEpi e{nullptr, nullptr, nullptr, nullptr, c->err.as<unsigned>(), c->wait_us};
     // launches of at most kMaxViews views, or hook->chunks launches
     const int step = hook ? std::min(kMaxViews, (nP + hook->chunks - 1) / hook->chunks)
@@ -170,7 +187,7 @@ mexct_status fp_run(mexct_ctx* c, const void* d_vol, int vt, int W, int H, float
       a->nviews = std::min(step, nP - v0);
       a->view0 = v0;
       for (int i = 0; i < a->nviews; ++i) trig_of(angles[v0 + i], &a->trig[i]);
-      MEXCT_TRY_CUDA(launch_fp_slab(geom, false, false, *a, mx, my, c->padx.p, c->pady.p, Pf, vt,
+      MEXCT_TRY_CUDA(launch_fp_slab(geom, false, false, *a, mx, my, c->padx.p, py, Pf, vt,
                                     d_out, ot, e, st),
                      "fp: launch");
       if (hook)
@@ -349,7 +366,9 @@ mexct_status fp_det_impl(mexct_ctx* c, const float* d_vol, int W, int H, float s
   int Pf = 0;
   const int ss = det->ss;
   // rows that are the volume's slices: the z-fastest kernel, as the standard FP
-  const bool rows = fp_uses_rows(geom) && ss == 1 && det->dv == 1.0f && det->det_h == H;
+  a->nviews = std::min(kMaxViews, nP);
+  for (int i = 0; i < a->nviews; ++i) trig_of(angles[i], &a->trig[i]);
+  const bool rows = ss == 1 && det->dv == 1.0f && det->det_h == H && fp_uses_rows(geom, *a, H, 0);
   mexct_status s = prepare_slab(c, d_vol, kF32, W, H, false, geom, rows, &mx, &my, &Pf, st);
   if (s) return s;
   const long long M = a->P * nP;
@@ -653,9 +672,11 @@ mexct_status osc_dev_impl(mexct_ctx* c, float* d_mu, int mu_type,
   // copies along with mu.
   CUtensorMap mx, my;
   int Pf = 0;
-  mexct_status ps = prepare_slab(c, d_mu, mu_type, W, H, /*border=*/true, geom, fp_uses_rows(geom),
-                                 &mx, &my, &Pf, st);
+  const bool rows = subset_uses_rows(geom, W, H, H, sad, angles, nP, nSub, 1);
+  mexct_status ps = prepare_slab(c, d_mu, mu_type, W, H, /*border=*/true, geom, rows, &mx, &my,
+                                 &Pf, st);
   if (ps) return ps;
+  void* py = rows ? nullptr : c->pady.p;
   std::unique_ptr<RayArgs> ra(new RayArgs);
   std::unique_ptr<VoxArgs> va(new VoxArgs);
   fill_std_rays(*ra, W, H, sad, geom, /*osc=*/true);
@@ -674,14 +695,14 @@ mexct_status osc_dev_impl(mexct_ctx* c, float* d_mu, int mu_type,
     if (nv > 0) {
       SlabEpi e{d_pre, d_post, c->r1.as<float>(), c->r2.as<float>(), c->err.as<unsigned>(),
                 c->wait_us};
-      MEXCT_TRY_CUDA(launch_fp_slab(geom, true, true, *ra, mx, my, c->padx.p, c->pady.p, Pf,
-                                    mu_type, nullptr, kF32, e, st),
+      MEXCT_TRY_CUDA(launch_fp_slab(geom, true, true, *ra, mx, my, c->padx.p, py, Pf, mu_type,
+                                    nullptr, kF32, e, st),
                      "osc_iter: fp");
     }
     // An empty subset still runs the update: num = den = 0 gives
     // max(mu + mu*0/0, 0) = 0 inside the circle, as in the reference.
     MEXCT_TRY_CUDA(launch_osc_bp_update(geom, *va, c->r1.as<float>(), c->r2.as<float>(),
-                                        d_mu, mu_type, c->padx.p, c->pady.p, Pf, st),
+                                        d_mu, mu_type, c->padx.p, py, Pf, st),
                    "osc_iter: bp/update");
   }
   return MEXCT_OK;

@@ -126,8 +126,9 @@ bool subset_order(int n, int first, int32_t* picks) {
 mexct_status enqueue_objective(mexct_osctv* s, cudaStream_t st) {
   CUtensorMap mx, my;
   int Pf = 0;
+  const bool rows = subset_uses_rows(s->geom, s->W, s->H, s->H, s->sad, s->angles.data(), s->nP, 1, 2);
   mexct_status ps = prepare_slab_bufs(s->padx, s->pady, s->err, s->mu.p, s->mu_type, s->W, s->H,
-                                      /*border=*/true, s->geom, fp_uses_rows(s->geom), &mx, &my, &Pf, st);
+                                      /*border=*/true, s->geom, rows, &mx, &my, &Pf, st);
   if (ps) return ps;
   std::unique_ptr<RayArgs> ra(new RayArgs);
   fill_std_rays(*ra, s->W, s->H, s->sad, s->geom, /*osc=*/true);
@@ -143,8 +144,8 @@ mexct_status enqueue_objective(mexct_osctv* s, cudaStream_t st) {
     for (int i = 0; i < nv; ++i) trig_of(s->angles[v0 + i], &ra->trig[i]);
     SlabEpi e{s->pre.as<float>(), s->post.as<float>(), nullptr, nullptr, s->err.as<unsigned>()};
     e.obj = s->objp.as<double>() + (size_t)v0 * tiles;
-    MEXCT_TRY_CUDA(launch_fp_slab_objective(s->geom, *ra, mx, my, s->padx.p, s->pady.p, Pf,
-                                            s->mu_type, e, st),
+    MEXCT_TRY_CUDA(launch_fp_slab_objective(s->geom, *ra, mx, my, s->padx.p,
+                                            rows ? nullptr : s->pady.p, Pf, s->mu_type, e, st),
                    "osctv: objective fp");
   }
   MEXCT_TRY_CUDA(launch_sum_partials(s->objp.as<double>(), (long long)s->nP * tiles,
@@ -169,9 +170,12 @@ mexct_status enqueue_iteration(mexct_osctv* s, bool k_gt1, int nsub,
   // rewrites the padded copies along with mu.
   CUtensorMap mx, my;
   int Pf = 0;
+  const bool rows =
+      subset_uses_rows(s->geom, s->W, s->H, s->H, s->sad, s->angles.data(), s->nP, nsub, 1);
   mexct_status ps = prepare_slab_bufs(s->padx, s->pady, s->err, s->mu.p, s->mu_type, s->W, s->H,
-                                      /*border=*/true, s->geom, fp_uses_rows(s->geom), &mx, &my, &Pf, st);
+                                      /*border=*/true, s->geom, rows, &mx, &my, &Pf, st);
   if (ps) return ps;
+  void* py = rows ? nullptr : s->pady.p;
   for (int si = 0; si < nsub; ++si) {
     const int sel = picks[si];
     const int nv = (sel < 0 || sel >= s->nP) ? 0 : (s->nP - 1 - sel) / nsub + 1;
@@ -187,12 +191,12 @@ mexct_status enqueue_iteration(mexct_osctv* s, bool k_gt1, int nsub,
       SlabEpi e{s->pre.as<float>(), s->post.as<float>(), s->r1.p, s->r2.p,
                 s->err.as<unsigned>()};
       e.rscale = std::ldexp(1.0f, -s->data_exp);
-      MEXCT_TRY_CUDA(launch_fp_slab(s->geom, true, true, *ra, mx, my, s->padx.p, s->pady.p, Pf,
+      MEXCT_TRY_CUDA(launch_fp_slab(s->geom, true, true, *ra, mx, my, s->padx.p, py, Pf,
                                     s->mu_type, nullptr, s->data_type, e, st),
                      "osctv: fp");
     }
     MEXCT_TRY_CUDA(launch_osc_bp_update(s->geom, *va, s->r1.p, s->r2.p, s->mu.p, s->mu_type,
-                                        s->padx.p, s->pady.p, Pf, st, s->data_type),
+                                        s->padx.p, py, Pf, st, s->data_type),
                    "osctv: bp/update");
   }
   (void)P;
@@ -292,7 +296,9 @@ mexct_status mexct_osctv_create_ex(mexct_ctx* ctx, const float* d_pre, const flo
   // and destroying solvers never synchronises the device (other streams keep
   // running); the caller's stream waits for the allocations.
   cudaStream_t a = s->own;
-  const FpLayout lay = fp_layout(fp_uses_rows(geom), W, H, mu_type);
+  // either kernel's layouts: the iterations' subset counts decide
+  FpLayout lay = fp_layout(false, W, H, mu_type);
+  if (geom != 2) lay.px = std::max(lay.px, fp_layout(true, W, H, mu_type).px);
   const size_t parts = std::max({tv_partials_needed(W, W, H), tv_fused_partials(W, W, H),
                                  ssd_partials_needed()}) + 8;
   // the fused TV keeps x in tvbuf (and tvx where rows are not whole) and its
@@ -353,19 +359,22 @@ mexct_status mexct_osctv_create_ex(mexct_ctx* ctx, const float* d_pre, const flo
     CUtensorMap mx, my;
     int Pf = 0;
     mexct_status ps = prepare_slab_bufs(s->padx, s->pady, s->err, s->mu.p, mu_type, W, H, true,
-                                        geom, fp_uses_rows(geom), &mx, &my, &Pf, st);
+                                        geom, /*rows=*/false, &mx, &my, &Pf, st);
     if (ps) return ps;
     std::unique_ptr<RayArgs> ra(new RayArgs);
     fill_std_rays(*ra, W, H, sad, geom, true);
     ra->nviews = 0;  // no work: sets attributes only
     SlabEpi e{s->pre.as<float>(), s->post.as<float>(), s->r1.p, s->r2.p, s->err.as<unsigned>()};
-    MEXCT_TRY_CUDA(launch_fp_slab(geom, true, true, *ra, mx, my, s->padx.p, s->pady.p, Pf,
-                                  mu_type, nullptr, data_type, e, st),
-                   "osctv_create: kernel setup");
-    e.obj = s->objp.as<double>();
-    MEXCT_TRY_CUDA(launch_fp_slab_objective(geom, *ra, mx, my, s->padx.p, s->pady.p, Pf, mu_type,
-                                            e, st),
-                   "osctv_create: kernel setup");
+    for (const void* py : {static_cast<const void*>(s->pady.p), static_cast<const void*>(nullptr)}) {
+      if (geom == 2 && !py) continue;  // parallel / fan: the rows kernel too
+      e.obj = nullptr;
+      MEXCT_TRY_CUDA(launch_fp_slab(geom, true, true, *ra, mx, my, s->padx.p, py, Pf, mu_type,
+                                    nullptr, data_type, e, st),
+                     "osctv_create: kernel setup");
+      e.obj = s->objp.as<double>();
+      MEXCT_TRY_CUDA(launch_fp_slab_objective(geom, *ra, mx, my, s->padx.p, py, Pf, mu_type, e, st),
+                     "osctv_create: kernel setup");
+    }
   }
   *out = s.release();
   return MEXCT_OK;

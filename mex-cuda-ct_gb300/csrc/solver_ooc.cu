@@ -249,8 +249,9 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
   }
   if ((size_t)(q - static_cast<unsigned char*>(db.p)) > total)
     return set_err(MEXCT_ERR_CUDA, "osc_tv_ooc: internal layout error");
-  const bool rows = fp_uses_rows(geom);  // one z-fastest layout, else two
-  const size_t pad_half = rows ? 0 : al(fp_layout(false, W, nz, kF32).px) / 4;  // floats
+  // of the iteration: one z-fastest layout (py null), else two
+  bool rows = false;
+  const size_t pad_half = al(fp_layout(false, W, nz, kF32).px) / 4;  // floats
 
   Streams S;
   MEXCT_TRY_CUDA(cudaStreamCreateWithFlags(&S.st, cudaStreamNonBlocking), "osc_tv_ooc: stream");
@@ -379,6 +380,7 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
     const int ns = nsubs[k - 1];
     const int32_t* pk = picks[k - 1].data();
     const int oth = 1 - cur;
+    rows = subset_uses_rows(geom, W, H, nz, sad, angles, nP, ns, 1);
     if (k == 2) {
       // OSC_TV_recon.m:41,62: from iteration 2 on, pre(1) = post(1) = 0
       MEXCT_TRY_CUDA(cudaStreamSynchronize(S.cin), "osc_tv_ooc: sync");
@@ -395,7 +397,7 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
       SlabIo io{hmu[cur], z0, z1, nullptr, nullptr};
       mexct_status e = run_slab(io, z0, z1, [&](int bs, const float**) -> mexct_status {
         float* px = Wk[bs];
-        float* py = Wk[bs] + pad_half;
+        float* py = rows ? nullptr : Wk[bs] + pad_half;
         MEXCT_TRY_CUDA(launch_pad_volume_sub(rows, X[bs], W, m, false, false, px, py, st, true),
                        "osc_tv_ooc: pad");
         return fp_part(px, py, z0, m, nv, i > 0);
@@ -421,7 +423,7 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
         SlabIo io{src, z0, z1, (last && k > 1) ? hmu[cur] : nullptr, hmu[oth]};
         mexct_status e = run_slab(io, z0, z1, [&](int bs, const float** out) -> mexct_status {
           float* px = Wk[bs];
-          float* py = Wk[bs] + pad_half;
+          float* py = rows ? nullptr : Wk[bs] + pad_half;
           MEXCT_TRY_CUDA(launch_pad_volume_sub(rows, X[bs], W, m, false, false, px, py, st, true),
                          "osc_tv_ooc: pad");
           fill_vox(*va, W, H, sad);

@@ -108,7 +108,9 @@ mexct_status fp_sub_impl(mexct_ctx* c, const float* d_slab, int W, int H, int z0
   a->zhi = (float)(rhi + 1);
   a->accum = accumulate ? 1 : 0;
   a->nall = nP;
-  const bool rows = fp_uses_rows(geom);
+  a->nviews = std::min(kMaxViews, nP);
+  for (int i = 0; i < a->nviews; ++i) trig_of(angles[i], &a->trig[i]);
+  const bool rows = fp_uses_rows(geom, *a, nz, 0);
   const FpLayout L = fp_layout(rows, W, nz, kF32);
   MEXCT_TRY_CUDA(c->padx.ensure_async(L.px, st), "fp_sub: workspace");
   MEXCT_TRY_CUDA(c->pady.ensure_async(L.py, st), "fp_sub: workspace");
@@ -127,8 +129,8 @@ mexct_status fp_sub_impl(mexct_ctx* c, const float* d_slab, int W, int H, int z0
     a->nviews = std::min(kMaxViews, nP - v0);
     a->view0 = v0;
     for (int i = 0; i < a->nviews; ++i) trig_of(angles[v0 + i], &a->trig[i]);
-    MEXCT_TRY_CUDA(launch_fp_slab_sub(geom, *a, mx, my, c->padx.p, c->pady.p, L.pitch, d_sino,
-                                      e, st),
+    MEXCT_TRY_CUDA(launch_fp_slab_sub(geom, *a, mx, my, c->padx.p, rows ? nullptr : c->pady.p,
+                                      L.pitch, d_sino, e, st),
                    "fp_sub: launch");
   }
   return MEXCT_OK;

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <limits>
+#include <memory>
 #include <vector>
 
 #include "../../include/mexct.h"
@@ -326,6 +327,24 @@ mexct_status mexct_autotune_fp(mexct_ctx* ctx, const void* d_vol, int vt, int W,
   if (s) return s;
   if (best) *best = b;
   if (best_ms) *best_ms = ms;
+  return MEXCT_OK;
+}
+
+mexct_status mexct_fp_plan(int W, int H, float sad, const float* angles, int nP, int geom,
+                           int nsub, int sms, int* rows, int* views, int* split) {
+  if (!angles || !rows || !views || !split) return set_err(MEXCT_ERR_ARG, "fp_plan: NULL pointer");
+  if (W <= 0 || H <= 0 || nP <= 0 || nsub < 0 || geom < 0 || geom > 2)
+    return set_err(MEXCT_ERR_ARG, "fp_plan: bad dims %d x %d x %d / geometry %d / subsets %d", W, H,
+                   nP, geom, nsub);
+  if (sms <= 0) sms = device_sms();
+  std::unique_ptr<RayArgs> a(new RayArgs);
+  fill_std_rays(*a, W, H, sad, geom, nsub > 0);
+  const int stride = std::max(nsub, 1), epi = nsub > 0 ? 1 : 0;
+  a->nall = (nP + stride - 1) / stride;
+  a->nviews = std::min(kMaxViews, a->nall);
+  for (int i = 0; i < a->nviews; ++i) trig_of(angles[(size_t)i * stride], &a->trig[i]);
+  *rows = fp_uses_rows(geom, *a, H, epi, sms) ? 1 : 0;
+  fp_rows_shape(geom, *a, epi, sms, views, split);
   return MEXCT_OK;
 }
 

@@ -35,6 +35,8 @@ _lib.register("mexct_shape_clear", [_P])
 _lib.register("mexct_autotune_fp", [_P, _P, _i, _i, _i, _f, _P, _i, _i, _P, _i, _P, _SP, _DP])
 _lib.register("mexct_autotune_bp", [_P, _P, _i, _i, _i, _i, _f, _P, _i, _P, _i, _P, _SP, _DP])
 
+_lib.register("mexct_fp_plan", [_i, _i, _f, _P, _i, _i, _i, _i] + [ctypes.POINTER(_i)] * 3)
+
 _CODES = {"float32": _lib.F32, "float16": _lib.F16, "bfloat16": _lib.BF16}
 
 
@@ -96,3 +98,13 @@ def autotune_fp(vol, sad, angles, geom, out=None, out_dtype=None, stream=None):
               nP, _geom_flag(geom), _dptr(out), _dtype_code(out), _stream(stream),
               ctypes.byref(s), ctypes.byref(ms))
     return out, s.as_dict(), ms.value
+
+
+def fp_plan(W, H, sad, angles, geom, nsub=0, sms=0):
+    """(rows, views, split) of a parallel / fan FP (nsub = 0) or OSC iteration: rows False is
+    the slab kernel; sms: SM count to plan for (0: the current device's)."""
+    a = _angles(angles, 0)
+    r, v, s = _i(), _i(), _i()
+    _lib.call("mexct_fp_plan", int(W), int(H), float(sad), _ptr(a), a.size, _geom_flag(geom),
+              int(nsub), int(sms), ctypes.byref(r), ctypes.byref(v), ctypes.byref(s))
+    return bool(r.value), v.value, s.value
