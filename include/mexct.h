@@ -436,6 +436,12 @@ mexct_status mexct_fp_plan(int W, int H, float sad, const float* angles, int nP,
                            int geom, int nsub, int sms, int* rows, int* views,
                            int* split);
 
+/* Which form the FP32 TV descent of an Nx x Ny x Nz volume takes outside stream
+ * capture (16-byte aligned volumes; sms as above): *fused = 1 one sweep per step
+ * (three workspace volumes, four where Nx % 4 != 0), 0 a norm and an update sweep
+ * (one). */
+mexct_status mexct_tv_plan(int Nx, int Ny, int Nz, int n_steps, int sms, int* fused);
+
 /* ---- allocation-free variant ------------------------------------------ */
 
 /* TV descent for callers that cannot allocate device memory while they run.

@@ -622,6 +622,25 @@ bool tv_fused_ok(int Nx, int Ny, int Nz) {
          (long long)tvf_pitch(Nx) * Ny * ((long long)Nz + 2) < (1LL << 31);
 }
 
+// Whether the fused steps are the faster form.  Rows that are not whole: always
+// (the pair would be the scalar tv_sweep).  Else the pair's tiles of 124 x 15
+// columns stand against tiles of 128 x 7, which cost half as much each and move
+// more memory: once the pair fills two CTAs on most SMs, a step of the pair takes
+// 1.95 times the tiles' ratio of a fused step's time, and the first and last sweep
+// of a fused descent add 0.2 steps.  So the columns that the tiles waste decide:
+// 20 steps, pair and fused, 512^3 10.95 and 9.95 ms, 384^3 5.36 and 4.46, but 600^2
+// x 300 7.38 and 8.15, 372 x 360 x 200 2.15 and 2.48; one step, 512^3 547 and 587
+// us.  Below that the pair's latency counts: 256^2 x 16 0.54 and 0.25 ms, 248 x 240
+// x 240 1.40 and 1.20.
+bool tv_fused_pays(int Nx, int Ny, int Nz, int n_steps, bool whole, int sms) {
+  if (!whole) return true;
+  if (sms <= 0) sms = device_sms();
+  const long long pair = (long long)((Nx + kT4Ox - 1) / kT4Ox) * ((Ny + kT4Oy - 1) / kT4Oy);
+  const long long fused = (long long)((Nx + 127) / 128) * std::max(1, (Ny - 1 + kTfOy - 1) / kTfOy);
+  if (pair * ((Nz + kT4Z - 1) / kT4Z) * 100 <= 185ll * sms) return true;
+  return (n_steps + 0.2) * (double)fused <= 1.95 * n_steps * (double)pair;
+}
+
 template <int MODE, bool XVEC>
 static cudaError_t tvf_go(const TvFused& a, dim3 grd, cudaStream_t st) {
   const int wx = tvf_wx(a.Nx);

@@ -331,7 +331,10 @@ cudaError_t launch_tv_update(const void* x, void* y, int x_type, int Nx,
 // when Nx % 4 != 0 or in / out are not 16-byte aligned (else may be null).
 // scale2: two floats; partials: tv_fused_partials doubles; counter must be 0.
 // c is multiplied by *cmul (device) when cmul is not null.
+// tv_fused_pays: whether they beat the pair of sweeps (whole: rows and pointers
+// of whole 16-byte units; sms 0: the current device's).
 bool tv_fused_ok(int Nx, int Ny, int Nz);
+bool tv_fused_pays(int Nx, int Ny, int Nz, int n_steps, bool whole, int sms = 0);
 size_t tv_fused_elems(int Nx, int Ny, int Nz);
 size_t tv_fused_partials(int Nx, int Ny, int Nz);
 cudaError_t launch_tv_fused(const float* in, float* out, int Nx, int Ny, int Nz, float c,

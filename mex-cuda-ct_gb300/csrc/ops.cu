@@ -733,11 +733,12 @@ mexct_status tv_dev_impl(mexct_ctx* c, const void* d_in, int t, int Nx,
   MEXCT_TRY_CUDA(ensure_reduction(c, std::max(tv_partials_needed(Nx, Ny, Nz),
                                               tv_fused_partials(Nx, Ny, Nz))),
                  "tvmin3d: workspace");
-  if (t == kF32 && tv_fused_ok(Nx, Ny, Nz) && !capturing(st)) {
+  const bool whole = Nx % 4 == 0 && (((uintptr_t)d_in | (uintptr_t)d_out) & 15) == 0;
+  if (t == kF32 && tv_fused_ok(Nx, Ny, Nz) && tv_fused_pays(Nx, Ny, Nz, n_steps, whole) &&
+      !capturing(st)) {
     // One gradient per step; its three or four buffers may not fit where the
     // pair of sweeps below (one buffer) does.  A captured call cannot allocate:
     // it keeps to the buffer that any earlier call of the size has made.
-    const bool whole = Nx % 4 == 0 && (((uintptr_t)d_in | (uintptr_t)d_out) & 15) == 0;
     const size_t wb = tv_fused_elems(Nx, Ny, Nz) * sizeof(float);
     cudaError_t e = cudaSuccess;
     for (Buf* b : {&c->r1, &c->r2, &c->r3, &c->tvx})

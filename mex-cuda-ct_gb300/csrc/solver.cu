@@ -29,6 +29,8 @@
 
 using namespace mexct;
 
+static constexpr int kTvSteps = 20;  // CUDAmex_TVmin_3D.cu:221
+
 struct mexct_osctv {
   mexct_ctx* ctx = nullptr;
   int device = 0;
@@ -79,13 +81,13 @@ struct mexct_osctv {
   int tiles() const { return ((W + 31) / 32) * ((H + 7) / 8); }
   // two floats (the fused TV alternates between them)
   float* tv_scale() { return reinterpret_cast<float*>(scal.as<double>() + 1); }
-  bool fused_tv() const { return mu_type == kF32 && tv_fused_ok(W, W, H); }
+  bool fused_tv() const {
+    return mu_type == kF32 && tv_fused_ok(W, W, H) && tv_fused_pays(W, W, H, kTvSteps, W % 4 == 0);
+  }
   double* tv_norm() { return scal.as<double>() + 2; }
 };
 
 namespace {
-
-constexpr int kTvSteps = 20;  // CUDAmex_TVmin_3D.cu:221
 
 int num_subsets(int s_init, int s_final, double p, int max_iters, int k) {
   if (max_iters <= 1) return s_final;

@@ -35,6 +35,7 @@ _lib.register("mexct_shape_clear", [_P])
 _lib.register("mexct_autotune_fp", [_P, _P, _i, _i, _i, _f, _P, _i, _i, _P, _i, _P, _SP, _DP])
 _lib.register("mexct_autotune_bp", [_P, _P, _i, _i, _i, _i, _f, _P, _i, _P, _i, _P, _SP, _DP])
 
+_lib.register("mexct_tv_plan", [_i] * 5 + [ctypes.POINTER(_i)])
 _lib.register("mexct_fp_plan", [_i, _i, _f, _P, _i, _i, _i, _i] + [ctypes.POINTER(_i)] * 3)
 
 _CODES = {"float32": _lib.F32, "float16": _lib.F16, "bfloat16": _lib.BF16}
@@ -108,3 +109,10 @@ def fp_plan(W, H, sad, angles, geom, nsub=0, sms=0):
     _lib.call("mexct_fp_plan", int(W), int(H), float(sad), _ptr(a), a.size, _geom_flag(geom),
               int(nsub), int(sms), ctypes.byref(r), ctypes.byref(v), ctypes.byref(s))
     return bool(r.value), v.value, s.value
+
+
+def tv_plan(Nx, Ny, Nz, n_steps=20, sms=0):
+    """Whether an FP32 TV descent takes one sweep per step (else a norm and an update)."""
+    f = _i()
+    _lib.call("mexct_tv_plan", int(Nx), int(Ny), int(Nz), int(n_steps), int(sms), ctypes.byref(f))
+    return bool(f.value)
