@@ -659,7 +659,8 @@ cudaError_t launch_tv_fused(const float* in, float* out, int Nx, int Ny, int Nz,
   // whole, x_2, x_4, ... go to out); g_0, g_1, ... between work[1] and work[2]
   const bool whole = Nx % 4 == 0 && ((uintptr_t)in & 15) == 0 && ((uintptr_t)out & 15) == 0;
   float* xb[2] = {work[0], whole ? out : work[3]};
-  if (!xb[1]) return cudaErrorInvalidValue;
+  // (the last sweep would turn rows of gp voxels into rows of Nx in place)
+  if (!xb[1] || (!whole && xb[1] == out && n_steps % 2 != 0)) return cudaErrorInvalidValue;
   TvFused a{};
   a.gp = gp;
   a.Nx = Nx;

@@ -328,7 +328,8 @@ cudaError_t launch_tv_update(const void* x, void* y, int x_type, int Nx,
 // n_steps >= 1 whole TV steps of an FP32 volume, one gradient per step: in ->
 // out (which may be the same).  work: buffers of tv_fused_elems floats each
 // (16-byte aligned); [0] x, [1] and [2] gradients, [3] x again, needed only
-// when Nx % 4 != 0 or in / out are not 16-byte aligned (else may be null).
+// when Nx % 4 != 0 or in / out are not 16-byte aligned (else may be null); it
+// may be `out` where that has room and n_steps is even.
 // scale2: two floats; partials: tv_fused_partials doubles; counter must be 0.
 // c is multiplied by *cmul (device) when cmul is not null.
 // tv_fused_pays: whether they beat the pair of sweeps (whole: rows and pointers

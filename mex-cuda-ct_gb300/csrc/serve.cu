@@ -126,13 +126,9 @@ size_t mexct_request_bytes(const mexct_request* r) {
   const int nv = (r->nP + smin - 1) / smin;
   const size_t rs = r->data_type == MEXCT_F16 ? 2 : 4;
   const size_t quads = 2 * sino_pad_elems(r->W, r->H, nv) * 4 * rs;
-  // rows that are not a multiple of four voxels: the TV buffer's spare columns
-  // and a second one
-  const size_t tv = r->mu_type == MEXCT_F32 && r->W % 4 != 0
-                        ? 4 * (2 * tv_fused_elems(r->W, r->W, r->H) - N) : 0;
   // staging (pre, post, recon) + solver (pre, post, residual views, mu,
   // mu_old, TV buffer, two padded copies).
-  return 4 * (2 * M + N) + 4 * (2 * M) + quads + ds * (3 * N + 2 * pad) + tv + (1 << 20);
+  return 4 * (2 * M + N) + 4 * (2 * M) + quads + ds * (3 * N + 2 * pad) + (1 << 20);
 }
 
 mexct_status mexct_server_create(int device, int slots, size_t budget, mexct_server** out) {

@@ -41,7 +41,7 @@ struct mexct_osctv {
   int data_type = kF32, data_exp = 0;
   float sad = 0.f;
   std::vector<float> angles;
-  Buf mu, mu_old, pre, post, padx, pady, err, r1, r2, tvbuf, tvx, red, cnt, scal, objp;
+  Buf mu, mu_old, pre, post, padx, pady, err, r1, r2, tvbuf, red, cnt, scal, objp;
   int k_done = 0;
   bool pre_zeroed = false;
   bool obj_valid = false;  // the last iteration computed the objective
@@ -64,8 +64,8 @@ struct mexct_osctv {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   ~mexct_osctv() {
     for (auto& g : graphs) cudaGraphExecDestroy(g.second);
-    for (Buf* b : {&mu, &mu_old, &pre, &post, &padx, &pady, &err, &r1, &r2, &tvbuf, &tvx, &red, &cnt,
-                   &scal, &objp})
+    for (Buf* b : {&mu, &mu_old, &pre, &post, &padx, &pady, &err, &r1, &r2, &tvbuf, &red, &cnt, &scal,
+                   &objp})
       b->release();  // stream-ordered on `own`, after all its work
     if (ev_in) cudaEventDestroy(ev_in);
     if (ev_out) cudaEventDestroy(ev_out);
@@ -206,13 +206,14 @@ mexct_status enqueue_iteration(mexct_osctv* s, bool k_gt1, int nsub,
     MEXCT_TRY_CUDA(launch_ssd(s->mu_old.p, s->mu.p, s->mu_type, (long long)N, 1,
                               s->red.as<double>(), s->cnt.as<unsigned>(), s->d_a(), st),
                    "osctv: d_a");
-    // FP32: one gradient per step; the padded copies of mu are spent (the next
-    // iteration pads anew) and hold the gradients.  Otherwise 20 pairs of
-    // sweeps on (mu, tvbuf); an even count ends in mu.
+    // Fused: one gradient per step; the padded copies of mu are spent (the next
+    // iteration pads anew) and hold the gradients, tvbuf and mu the volumes
+    // between steps (an even count leaves the last of them in tvbuf).  Otherwise
+    // 20 pairs of sweeps on (mu, tvbuf); an even count ends in mu.
     const bool fused = s->fused_tv();
     if (fused) {
       float* work[4] = {s->tvbuf.as<float>(), s->padx.as<float>(), s->pady.as<float>(),
-                        s->tvx.as<float>()};
+                        s->mu.as<float>()};
       MEXCT_TRY_CUDA(launch_tv_fused(s->mu.as<float>(), s->mu.as<float>(), s->W, s->W, s->H, tvc,
                                      s->d_a(), kTvSteps, work, s->red.as<double>(),
                                      s->cnt.as<unsigned>(), s->tv_scale(), s->tv_norm(), st),
@@ -303,14 +304,12 @@ mexct_status mexct_osctv_create_ex(mexct_ctx* ctx, const float* d_pre, const flo
   if (geom != 2) lay.px = std::max(lay.px, fp_layout(true, W, H, mu_type).px);
   const size_t parts = std::max({tv_partials_needed(W, W, H), tv_fused_partials(W, W, H),
                                  ssd_partials_needed()}) + 8;
-  // the fused TV keeps x in tvbuf (and tvx where rows are not whole) and its
-  // gradients in the padded copies
+  // the fused TV keeps x in tvbuf and mu, in rows of a multiple of four voxels, and
+  // its gradients in the padded copies
   const size_t tvb = s->fused_tv() ? tv_fused_elems(W, W, H) * sizeof(float) : 0;
-  MEXCT_TRY_CUDA(s->mu.ensure_async(vb, a), "osctv_create: mu");
+  MEXCT_TRY_CUDA(s->mu.ensure_async(std::max(vb, tvb), a), "osctv_create: mu");
   MEXCT_TRY_CUDA(s->mu_old.ensure_async(vb, a), "osctv_create: mu_old");
   MEXCT_TRY_CUDA(s->tvbuf.ensure_async(std::max(vb, tvb), a), "osctv_create: tv");
-  if (tvb && W % 4 != 0)
-    MEXCT_TRY_CUDA(s->tvx.ensure_async(tvb, a), "osctv_create: tv");
   MEXCT_TRY_CUDA(s->padx.ensure_async(std::max(lay.px, tvb), a), "osctv_create: padded mu");
   MEXCT_TRY_CUDA(s->pady.ensure_async(std::max(lay.py, tvb), a), "osctv_create: padded mu");
   MEXCT_TRY_CUDA(s->pre.ensure_async(M * 4, a), "osctv_create: pre");
