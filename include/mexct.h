@@ -62,7 +62,12 @@ const char* mexct_version(void);
  * (or serialise calls on a shared one). */
 mexct_status mexct_ctx_create(int device, mexct_ctx** out);
 mexct_status mexct_ctx_destroy(mexct_ctx* ctx);
-/* Release the context's workspaces (they are re-created on demand). */
+/* Release the context's workspaces (they are re-created on demand).  Beside what
+ * its calls cannot do without, a context keeps buffers that only make them faster:
+ * the general3D BP's pair buffers (16 bytes per voxel) and the TV descent's gradients
+ * (two or three volumes), up to 4 GiB each; larger ones last for one call.  An
+ * allocation of the library that runs out of memory frees them and is tried again;
+ * an allocation of the caller's cannot, which is what trim is for. */
 mexct_status mexct_ctx_trim(mexct_ctx* ctx);
 
 /* Bounded waits (no counterpart in the reference).  The slab forward projector
@@ -77,6 +82,10 @@ mexct_status mexct_ctx_trim(mexct_ctx* ctx);
  * synchronising its stream); clear != 0 zeroes it. */
 mexct_status mexct_ctx_set_wait_limit(mexct_ctx* ctx, int us);
 mexct_status mexct_ctx_device_errors(mexct_ctx* ctx, unsigned* flags, int clear);
+
+/* Diagnostics: the next n device allocations of the library, in any thread,
+ * report out of memory (0: none). */
+mexct_status mexct_fail_allocs(int n);
 
 /* ---- MEX-equivalent host entry points --------------------------------- */
 

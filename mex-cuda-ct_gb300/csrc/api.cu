@@ -4,10 +4,13 @@
 // per-view geometry tables, view chunking and the host<->device boundary of
 // the MEX-equivalent entry points.  All compute runs in the kernels of
 // k_proj.cu / k_iter.cu; there is no CPU fallback.
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -71,7 +74,49 @@ void Buf::release_synced() {
   release();
 }
 
-cudaError_t Buf::ensure_async(size_t bytes, cudaStream_t st) {
+// Contexts by device, for device_alloc; a failure to inject in the next
+// allocations (mexct_fail_allocs).
+static std::mutex g_live_mu;
+static std::vector<mexct_ctx*> g_live;
+static std::atomic<int> g_fail{0};
+
+// Frees the optional buffers of the current device's contexts (those in use by
+// another thread's call keep theirs); whether there were any.
+static bool give_back() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  bool any = false;
+  std::lock_guard<std::mutex> lk(g_live_mu);
+  for (mexct_ctx* c : g_live) {
+    if (c->device != dev) continue;
+    std::unique_lock<std::recursive_mutex> own(c->mu, std::try_to_lock);
+    if (!own.owns_lock()) continue;
+    for (Buf* b : c->optional_bufs()) {
+      any |= b->p != nullptr;
+      b->release_synced();
+    }
+  }
+  return any;
+}
+
+cudaError_t device_alloc(const std::function<cudaError_t()>& alloc, cudaStream_t st,
+                         bool optional) {
+  auto once = [&] {
+    int n = g_fail.load();
+    while (n > 0 && !g_fail.compare_exchange_weak(n, n - 1)) {
+    }
+    return n > 0 ? cudaErrorMemoryAllocation : alloc();
+  };
+  cudaError_t e = once();
+  if (e == cudaErrorMemoryAllocation && !optional && !capturing(st)) {
+    cudaGetLastError();
+    if (give_back()) e = once();
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
+cudaError_t Buf::ensure_async(size_t bytes, cudaStream_t st, bool optional) {
   if (bytes <= n && p) return cudaSuccess;
   if (p && is_async && ast != st) {
     // The old block was allocated on another stream, which may be a caller's
@@ -98,11 +143,10 @@ cudaError_t Buf::ensure_async(size_t bytes, cudaStream_t st) {
   }
   release();
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMallocAsync(&p, bytes, st);
+  cudaError_t e = device_alloc([&] { return cudaMallocAsync(&p, bytes, st); }, st, optional);
   if (e != cudaSuccess) {
     p = nullptr;
     n = 0;
-    cudaGetLastError();
     return e;
   }
   n = bytes;
@@ -115,11 +159,10 @@ cudaError_t Buf::ensure(size_t bytes) {
   if (bytes <= n && p) return cudaSuccess;
   release();
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc(&p, bytes);
+  cudaError_t e = device_alloc([&] { return cudaMalloc(&p, bytes); });
   if (e != cudaSuccess) {
     p = nullptr;
     n = 0;
-    cudaGetLastError();
     return e;
   }
   n = bytes;
@@ -243,6 +286,10 @@ mexct_status mexct_ctx_create(int device, mexct_ctx** out) {
     delete c;
     return cuda_err(e, "ctx_create: stream");
   }
+  {
+    std::lock_guard<std::mutex> lk(g_live_mu);
+    g_live.push_back(c);
+  }
   *out = c;
   return MEXCT_OK;
 }
@@ -261,6 +308,11 @@ mexct_status mexct_ctx_trim(mexct_ctx* c) {
     cudaFreeArray(c->tex_arr);
     c->tex_arr = nullptr;
   }
+  return MEXCT_OK;
+}
+
+mexct_status mexct_fail_allocs(int n) {
+  g_fail.store(n < 0 ? 0 : n);
   return MEXCT_OK;
 }
 
@@ -295,6 +347,10 @@ mexct_status mexct_ctx_destroy(mexct_ctx* c) {
     std::lock_guard<std::mutex> lk(g_default_mu);
     for (auto& d : g_default)
       if (d == c) d = nullptr;
+  }
+  {
+    std::lock_guard<std::mutex> lk(g_live_mu);
+    g_live.erase(std::remove(g_live.begin(), g_live.end(), c), g_live.end());
   }
   int prev = 0;
   cudaGetDevice(&prev);

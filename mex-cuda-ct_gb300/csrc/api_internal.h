@@ -30,7 +30,8 @@ struct Buf {
   // Stream-ordered allocation (cudaMallocAsync): no device-wide
   // synchronisation on allocation or release, so work on other streams keeps
   // running.  The buffer is released with cudaFreeAsync on the same stream.
-  cudaError_t ensure_async(size_t bytes, cudaStream_t st);
+  // optional: a failure takes nothing back from the contexts (device_alloc).
+  cudaError_t ensure_async(size_t bytes, cudaStream_t st, bool optional = false);
   // Free in the order of the stream the block was allocated on (that stream
   // must still exist: the owner's own stream).
   void release();
@@ -52,6 +53,18 @@ struct NvtxRange {
   NvtxRange(const NvtxRange&) = delete;
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
+
+// An allocation of the library.  Where it runs out of memory, what the contexts
+// of the device keep for speed alone (mexct_ctx::optional_bufs) is freed and it is
+// tried once more, unless it is itself optional or st is being captured.
+cudaError_t device_alloc(const std::function<cudaError_t()>& alloc, cudaStream_t st = nullptr,
+                         bool optional = false);
+// Optional buffers above this size are freed when their call has used them, in the
+// order of its stream (smaller ones are kept: 256^3 pair buffers 0.27 GB, 512^3 2.1).
+// tv_call_fused and g3d_bp_pairs allow for the allocations that this costs.
+constexpr size_t kKeepOptional = (size_t)4 << 30;
+
+bool tv_call_fused(int Nx, int Ny, int Nz, int n_steps, bool whole, int sms = 0);
 
 // Whether st is being captured (an unknown state counts as captured).
 bool capturing(cudaStream_t st);
@@ -88,9 +101,11 @@ struct mexct_ctx {
   mexct::Buf spad;   // padded sinogram views for BP
   mexct::Buf bpart;  // BP view-block partial sums
   mexct::Buf subs;   // one sub-ray sinogram of a super-sampled FP
-  mexct::Buf gpair;  // general3D BP: pair buffers, and the end of their last use
+  // Kept for speed alone (each user has a form without): general3D BP's pair
+  // buffers with the end of their last use; the fused TV's gradients and, for rows
+  // that are not whole, second volume.  Captured calls do not use them.
+  mexct::Buf gpair, tvw;
   cudaEvent_t gpair_ev = nullptr;
-  mexct::Buf tvx;    // TV: a second volume between steps (rows that are not whole)
   // Launch shapes: MEXCT_TUNE_* mode and the per-class table.
   int tune_mode = MEXCT_TUNE_HEURISTIC;
   // Limit of one bounded wait in the slab FP (SlabEpi::wait_us encoding).
@@ -121,8 +136,9 @@ struct mexct_ctx {
 
   std::vector<mexct::Buf*> all_bufs() {
     return {&in, &in2, &in3, &out, &volT, &r1, &r2, &r3, &tabs, &red, &cnt, &scal,
-            &padx, &pady, &err, &spad, &bpart, &subs, &tvx, &gpair};
+            &padx, &pady, &err, &spad, &bpart, &subs, &tvw, &gpair};
   }
+  std::vector<mexct::Buf*> optional_bufs() { return {&tvw, &gpair}; }
 };
 
 namespace mexct {

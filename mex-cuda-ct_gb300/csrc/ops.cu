@@ -55,7 +55,9 @@ mexct_status fp_tex(mexct_ctx* c, const float* d_vol, int W, int H, int geom,
     c->tex = 0;
     c->tex_arr = nullptr;
     cudaChannelFormatDesc ch = cudaCreateChannelDesc<float>();
-    MEXCT_TRY_CUDA(cudaMalloc3DArray(&c->tex_arr, &ch, make_cudaExtent(W, W, H), 0),
+    MEXCT_TRY_CUDA(device_alloc([&] {
+                     return cudaMalloc3DArray(&c->tex_arr, &ch, make_cudaExtent(W, W, H), 0);
+                   }, st),
                    "fp(texture): 3D array");
     cudaResourceDesc rd;
     std::memset(&rd, 0, sizeof rd);
@@ -508,10 +510,24 @@ mexct_status g3d_bp_dev_impl(mexct_ctx* c, const float* d_sino, int W, int H,
     if (!c->gpair_ev)
       MEXCT_TRY_CUDA(cudaEventCreateWithFlags(&c->gpair_ev, cudaEventDisableTiming), "g3d_bp: event");
     MEXCT_TRY_CUDA(cudaStreamWaitEvent(st, c->gpair_ev, 0), "g3d_bp: wait");
-    const cudaError_t e = c->gpair.ensure_async(4 * N * sizeof(float), st);
+    const cudaError_t e = c->gpair.ensure_async(4 * N * sizeof(float), st, /*optional=*/true);
     if (e == cudaErrorMemoryAllocation) pairs = false;
     else if (e != cudaSuccess) return cuda_err(e, "g3d_bp: workspace");
   }
+  // the end of the buffers' use, also where a launch failed; a large pair goes
+  // (it was allocated by this call, on st)
+  struct PairUse {
+    mexct_ctx* c;
+    cudaStream_t st;
+    cudaError_t end() {
+      if (!c) return cudaSuccess;
+      const cudaError_t e = cudaEventRecord(c->gpair_ev, st);
+      if (c->gpair.n > kKeepOptional) c->gpair.release();
+      c = nullptr;
+      return e;
+    }
+    ~PairUse() { end(); }
+  } use{pairs ? c : nullptr, st};
   float* acc = pairs ? c->gpair.as<float>() : d_vol;
   MEXCT_TRY_CUDA(cudaMemsetAsync(acc, 0, (pairs ? 4 : 1) * N * sizeof(float), st), "g3d_bp: zero");
   std::unique_ptr<RayArgs> a(new RayArgs);
@@ -526,7 +542,7 @@ mexct_status g3d_bp_dev_impl(mexct_ctx* c, const float* d_sino, int W, int H,
   }
   if (pairs) {
     MEXCT_TRY_CUDA(launch_g3d_bp_fold(acc, S, Z, d_vol, st), "g3d_bp: fold");
-    MEXCT_TRY_CUDA(cudaEventRecord(c->gpair_ev, st), "g3d_bp: event");
+    MEXCT_TRY_CUDA(use.end(), "g3d_bp: event");
   }
   return MEXCT_OK;
 }
@@ -708,6 +724,22 @@ mexct_status osc_dev_impl(mexct_ctx* c, float* d_mu, int mu_type,
   return MEXCT_OK;
 }
 
+}  // namespace
+
+namespace mexct {
+// Whether an FP32 TV call takes the fused steps.  Buffers that are not kept cost
+// ~2.2 ms per GB and call to allocate: more than whole rows gain (1000^2 x 700, 20
+// steps: pair 50 ms, fused 52 with kept buffers and 64 without), and other rows
+// need some ten steps (1001^2 x 560, 20 steps: 74, 43 and 57 ms; one: 3.7, 3.1, 17).
+bool tv_call_fused(int Nx, int Ny, int Nz, int n_steps, bool whole, int sms) {
+  if (!tv_fused_ok(Nx, Ny, Nz) || !tv_fused_pays(Nx, Ny, Nz, n_steps, whole, sms)) return false;
+  const size_t wb = tv_fused_elems(Nx, Ny, Nz) * sizeof(float);
+  return (whole ? 2 : 3) * wb <= kKeepOptional || (!whole && n_steps >= 10);
+}
+}  // namespace mexct
+
+namespace {
+
 // ---------------------------------------------------------------------------
 // TV descent: n_steps of (norm, update) on a ping-pong pair whose last write
 // lands in d_out.
@@ -734,28 +766,26 @@ mexct_status tv_dev_impl(mexct_ctx* c, const void* d_in, int t, int Nx,
                                               tv_fused_partials(Nx, Ny, Nz))),
                  "tvmin3d: workspace");
   const bool whole = Nx % 4 == 0 && (((uintptr_t)d_in | (uintptr_t)d_out) & 15) == 0;
-  if (t == kF32 && tv_fused_ok(Nx, Ny, Nz) && tv_fused_pays(Nx, Ny, Nz, n_steps, whole) &&
-      !capturing(st)) {
-    // One gradient per step; its three or four buffers may not fit where the
-    // pair of sweeps below (one buffer) does.  A captured call cannot allocate:
-    // it keeps to the buffer that any earlier call of the size has made.
+  if (t == kF32 && tv_call_fused(Nx, Ny, Nz, n_steps, whole) && !capturing(st)) {
+    // One gradient per step; the two or three further buffers may not fit where
+    // the pair of sweeps below (one buffer) does.  A captured call cannot
+    // allocate: it keeps to the buffer that any earlier call of the size has made.
     const size_t wb = tv_fused_elems(Nx, Ny, Nz) * sizeof(float);
-    cudaError_t e = cudaSuccess;
-    for (Buf* b : {&c->r1, &c->r2, &c->r3, &c->tvx})
-      if (e == cudaSuccess && (b != &c->tvx || !whole)) e = b->ensure(wb);
+    cudaError_t e = c->r1.ensure(wb);  // (before tvw, which it may give back)
+    if (e == cudaSuccess) e = c->tvw.ensure_async((whole ? 2 : 3) * wb, st, /*optional=*/true);
     if (e == cudaSuccess) {
-      float* work[4] = {c->r1.as<float>(), c->r2.as<float>(), c->r3.as<float>(),
-                        whole ? nullptr : c->tvx.as<float>()};
-      MEXCT_TRY_CUDA(launch_tv_fused((const float*)d_in, (float*)d_out, Nx, Ny, Nz, cval, nullptr,
-                                     n_steps, work, c->red.as<double>(), c->cnt.as<unsigned>(),
-                                     c->scal.as<float>(),
-                                     reinterpret_cast<double*>(c->scal.as<char>() + 8), st),
-                     "tvmin3d: steps");
+      float* w = c->tvw.as<float>();
+      const size_t n = wb / sizeof(float);
+      float* work[4] = {c->r1.as<float>(), w, w + n, whole ? nullptr : w + 2 * n};
+      const cudaError_t le = launch_tv_fused(
+          (const float*)d_in, (float*)d_out, Nx, Ny, Nz, cval, nullptr, n_steps, work,
+          c->red.as<double>(), c->cnt.as<unsigned>(), c->scal.as<float>(),
+          reinterpret_cast<double*>(c->scal.as<char>() + 8), st);
+      if (c->tvw.n > kKeepOptional) c->tvw.release();  // of this call, on st
+      MEXCT_TRY_CUDA(le, "tvmin3d: steps");
       return MEXCT_OK;
     }
     if (e != cudaErrorMemoryAllocation) return cuda_err(e, "tvmin3d: workspace");
-    cudaGetLastError();
-    for (Buf* b : {&c->r2, &c->r3, &c->tvx}) b->release_synced();
   }
   MEXCT_TRY_CUDA(c->r1.ensure(bytes), "tvmin3d: workspace");
   const void* src = d_in;

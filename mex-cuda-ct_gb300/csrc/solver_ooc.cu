@@ -212,7 +212,8 @@ mexct_status osc_tv_recon_ooc(mexct_ctx* ctx, const float* pre, const float* pos
   const SetLayout L = set_layout(W, nz);
   const size_t total = pl.bytes;
   DevBlock db;
-  MEXCT_TRY_CUDA(cudaMalloc(&db.p, total), "osc_tv_ooc: device memory");
+  MEXCT_TRY_CUDA(device_alloc([&] { return cudaMalloc(&db.p, total); }),
+                 "osc_tv_ooc: device memory");
   unsigned char* q = static_cast<unsigned char*>(db.p);
   auto carve = [&](size_t b) {
     unsigned char* r = q;

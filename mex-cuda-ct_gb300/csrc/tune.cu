@@ -352,7 +352,7 @@ mexct_status mexct_tv_plan(int Nx, int Ny, int Nz, int n_steps, int sms, int* fu
   if (!fused) return set_err(MEXCT_ERR_ARG, "tv_plan: NULL pointer");
   if (Nx <= 0 || Ny <= 0 || Nz <= 0 || n_steps <= 0)
     return set_err(MEXCT_ERR_ARG, "tv_plan: bad dims %d x %d x %d / steps %d", Nx, Ny, Nz, n_steps);
-  *fused = tv_fused_ok(Nx, Ny, Nz) && tv_fused_pays(Nx, Ny, Nz, n_steps, Nx % 4 == 0, sms) ? 1 : 0;
+  *fused = tv_call_fused(Nx, Ny, Nz, n_steps, Nx % 4 == 0, sms) ? 1 : 0;
   return MEXCT_OK;
 }
 

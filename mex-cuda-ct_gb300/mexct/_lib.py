@@ -92,6 +92,7 @@ SIGNATURES = {
     "mexct_vff_write": [_c.c_char_p, _P, _c.POINTER(_i), _F, _i],
     "mexct_fp_slab_occupancy": [_c.POINTER(_i)],
     "mexct_ctx_set_wait_limit": [_P, _i],
+    "mexct_fail_allocs": [_i],
     "mexct_ctx_device_errors": [_P, _c.POINTER(_c.c_uint), _i],
 }
 _RESTYPES = {"mexct_last_error": _c.c_char_p, "mexct_version": _c.c_char_p}
