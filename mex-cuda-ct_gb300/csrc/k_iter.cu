@@ -10,9 +10,10 @@
 //   tv_update_kernel gradient recomputed, y = x + scale*g into the other
 //                    buffer of a ping-pong pair.
 // Algorithmic traffic is 12 bytes per voxel per step (read x twice, write y).
-// Whole FP32 descents take tv_fused_kernel instead: one sweep and one gradient
-// per step.  The pair serves FP16 / BF16, the sub-volume sweeps and the
-// allocation-free form (one scratch volume).
+// Whole FP32 descents take tv_fused_kernel instead, one sweep and one gradient
+// per step, where that is faster (tv_fused_pays).  The pair serves the others,
+// FP16 / BF16, captured calls, the sub-volume sweeps and the allocation-free form
+// (one scratch volume).
 // FP32 volumes whose x extent is a multiple of 4 use tv4_kernel (four x-voxels
 // per thread, 16-byte loads and stores, packed FP32x2 arithmetic): 512^3 step
 // 0.92 -> 0.55 ms, 2.9 TB/s of algorithmic traffic; other volumes tv_sweep.
@@ -244,8 +245,9 @@ __device__ __forceinline__ V4 fma4(V4 a, V4 b, V4 c) {
 
 // 1 / (eps + |(a, b, c)|) of four voxels by the hardware reciprocal square root
 // and reciprocal: |.| = s2 rsqrt(s2).  s2 starts from FLT_MIN (no effect beside
-// eps), so both arguments are normal and the flush-to-zero forms give what
-// rsqrtf and a division of 1 give, without their range tests.
+// eps), so both arguments are normal and the flush-to-zero forms need no range
+// tests.  Each is within its documented error (a few ulp; 1 / x would be correctly
+// rounded): the tests hold whole steps to 1e-5 of the oracle.
 __device__ __forceinline__ float rsqrt_normal(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -1155,7 +1157,7 @@ __global__ void __launch_bounds__(256) prefilter_tiled_kernel(
 // the larger one: each row is scaled by the power of two that brings its largest
 // magnitude into [1, 2) and back at the store (exact, so a pair of like rows
 // gives the bits that it gives unscaled; without it a row beside one 1e4 times
-// larger was off by 4e-4; 15 us of 502 at 384^2 x 512).  A row of zeros stores
+// larger was off by 4e-4; 12 us of 499 at 384^2 x 512).  A row of zeros stores
 // zeros.
 //
 // A row with a value that is not finite or above 1e30 would reach its partner
@@ -1280,14 +1282,15 @@ __device__ __forceinline__ float prefilter_fast_input(const FiltArgs& A, float s
 
 // 2^-e and 2^e of a row's largest magnitude m = 2^e (1 .. 2), e >= -126; for a
 // row of zeros 2^e is 0.
-__device__ __forceinline__ unsigned row_exp(float m) {
-  return min(max(__float_as_uint(m) >> 23, 1u), 253u);
-}
-__device__ __forceinline__ float row_scale(float m) {
+// Magnitudes as their bits, which integers order alike (a NaN, whose row is kept out
+// of the transform, above all others).
+__device__ __forceinline__ unsigned magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned row_exp(unsigned m) { return min(max(m >> 23, 1u), 253u); }
+__device__ __forceinline__ float row_scale(unsigned m) {
   return __uint_as_float((254u - row_exp(m)) << 23);
 }
-__device__ __forceinline__ float row_unscale(float m) {
-  return m > 0.f ? __uint_as_float(row_exp(m) << 23) : 0.f;
+__device__ __forceinline__ float row_unscale(unsigned m) {
+  return m ? __uint_as_float(row_exp(m) << 23) : 0.f;
 }
 
 constexpr int kFftThreads = 256, kFftElems = 16 * kFftThreads;  // complex elements per CTA
@@ -1302,7 +1305,8 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   __shared__ float2 sm[kFftElems + kFftElems / 8];
   __shared__ int bad[2 * NF];  // rows kept out of the transform
   constexpr int TW = TF < 32 ? TF : 32, NWF = TF / TW;  // lanes and warps per transform
-  __shared__ float2 psum[NF * NWF], pmax[NF * NWF], edge[8 * NF * NWF];
+  __shared__ float2 psum[NF * NWF], edge[8 * NF * NWF];
+  __shared__ uint2 pmax[NF * NWF];
   // after the spatial kernel: the differences' spectrum and the twiddles
   const float2* spec = reinterpret_cast<const float2*>(kern + N);
   const float2 *tw1 = spec + N, *tw2 = tw1 + 4 * TF;
@@ -1357,18 +1361,19 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   // row sums and largest magnitudes, and each element's left neighbour: lane n -
   // 1, whose warp leaves its last lane's elements in edge
   const int wq = q * NWF + n / TW;
-  float2 sum = make_float2(0.f, 0.f), big = sum, left[8];
+  float2 sum = make_float2(0.f, 0.f), left[8];
+  uint2 big = make_uint2(0u, 0u);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     sum = c_add(sum, e[j]);
-    big = make_float2(fmaxf(big.x, fabsf(e[j].x)), fmaxf(big.y, fabsf(e[j].y)));
+    big = make_uint2(max(big.x, magnitude(e[j].x)), max(big.y, magnitude(e[j].y)));
   }
+  const unsigned lanes = TW == 32 ? 0xffffffffu : ((1u << (TW & 31)) - 1u) << (threadIdx.x & 31 & ~(TW - 1));
+  big = make_uint2(__reduce_max_sync(lanes, big.x), __reduce_max_sync(lanes, big.y));
 #pragma unroll
   for (int o = TW / 2; o > 0; o >>= 1) {
     sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
     sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
-    big.x = fmaxf(big.x, __shfl_xor_sync(0xffffffffu, big.x, o));
-    big.y = fmaxf(big.y, __shfl_xor_sync(0xffffffffu, big.y, o));
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -1387,11 +1392,11 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   const bool bad0 = bad[2 * q] != 0, bad1 = bad[2 * q + 1] != 0;
   // 2^-e of both rows, or 2^e (back); read again at the store instead of kept
   auto scales = [&](bool back) {
-    float2 m = pmax[q * NWF];
+    uint2 m = pmax[q * NWF];
 #pragma unroll
     for (int w = 1; w < NWF; ++w) {
-      const float2 b = pmax[q * NWF + w];
-      m = make_float2(fmaxf(m.x, b.x), fmaxf(m.y, b.y));
+      const uint2 b = pmax[q * NWF + w];
+      m = make_uint2(max(m.x, b.x), max(m.y, b.y));
     }
     return back ? make_float2(row_unscale(m.x), row_unscale(m.y))
                 : make_float2(row_scale(m.x), row_scale(m.y));
@@ -1487,13 +1492,15 @@ __global__ void __launch_bounds__(kFftThreads, 3) prefilter_fft_kernel(
   twiddle<R1, true>(e, w1);
   dft<R1, true>(e);
   const float db = live ? __ldg(dbeta + view) : 0.f;
-  const float2 unscale = scales(true);
+  // one factor: where it underflows, so does what it scales
+  float2 back = scales(true);
+  back = make_float2(back.x * db, back.y * db);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int u = n + j * TF;
     if (live && u < W) {
-      if (!bad0) out[row0 + u] = e[j].x * unscale.x * db;
-      if (two && !bad1) out[row0 + W + u] = e[j].y * unscale.y * db;
+      if (!bad0) out[row0 + u] = e[j].x * back.x;
+      if (two && !bad1) out[row0 + W + u] = e[j].y * back.y;
     }
   }
   if (any) {  // rows kept out: the direct sum, from staged inputs (out may be sino)
