@@ -402,7 +402,7 @@ typedef struct mexct_shape {
 #define MEXCT_OP_BP 1
 
 /* Modes for a class without a table entry. */
-#define MEXCT_TUNE_FIXED 0     /* FP slab kernel; BP zc 16, rows 8, 1 view block */
+#define MEXCT_TUNE_FIXED 0     /* FP slab / rows kernel; BP zc 16, rows 8, 1 view block */
 #define MEXCT_TUNE_HEURISTIC 1 /* default: view blocks so small volumes fill the GPU */
 #define MEXCT_TUNE_AUTO 2      /* the first call of the class times every candidate
                                   shape on its own data and keeps the fastest (a call

@@ -2,7 +2,7 @@
 // MEXCT_FP_RAY and MEXCT_FP_TEXTURE variants), voxel-driven backprojectors
 // (standard BP, OSC dual BP + update, batched BP) and the general3D scatter
 // backprojector for sm_103a.  The standard and OSC forward projections run
-// in k_slab.cu (cone) and k_rows.cu (parallel, fan).
+// in k_slab.cu (cone; parallel, fan of few slices) and k_rows.cu (parallel, fan).
 //
 // Ray-per-thread FP (CUDAmex_FP.cu:56-346, CUDAmex_general3D_FP.cu:59-150)
 //   One thread per detector pixel; a warp owns 32 consecutive pixels of one
@@ -1095,8 +1095,8 @@ cudaError_t launch_g3d_bp(const RayArgs& a, const float* sino,
 
 // ---------------------------------------------------------------------------
 // OSC kernels.  The subset FP with the residual epilogue
-// (CUDAmex_oscIter.cu:140-271) is the slab kernel of k_slab.cu (cone) or the
-// rows kernel of k_rows.cu with border addressing and step 0.5.
+// (CUDAmex_oscIter.cu:140-271) is the slab kernel of k_slab.cu or the rows kernel
+// of k_rows.cu with border addressing and step 0.5.
 // ---------------------------------------------------------------------------
 // Dual BP of the residuals with border addressing (CUDAmex_oscIter.cu:305-356)
 // into register accumulators, then mu <- max(mu + mu*num/den, 0) inside the

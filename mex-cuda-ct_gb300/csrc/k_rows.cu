@@ -25,17 +25,21 @@
 // plane for 128 rows.  Measured, slab kernel -> this: 384^3 x 512 parallel
 // 52.4 -> 13.4 ms, fan 55.1 -> 14.7 ms; 243^2 x 201 x 361 fan in FP16 9.8 ->
 // 3.1 ms; 128^2 x 100 x 360 1.27 -> 0.60 ms; 64^3 x 90 0.107 -> 0.074 ms.
-// Error against 64 bits 2.3e-6 -> 3.7e-7 (shorter sums).  Bound now: about
-// half the issue slots (the weights a fifth of them), 16 warps per SM
-// waiting on shared memory and fixed latencies (23 % warps active).  Also
+// Volumes of few slices keep the slab kernel (fp_uses_rows).  Error against 64
+// bits 2.3e-6 -> 3.7e-7 (shorter sums).  Bound now (four views per CTA): 54 % of
+// the issue slots (the weights a fifth of them) and 60 % of the shared / L1 data
+// path at 16 warps per SM, which wait on fixed latencies and shared memory.  Also
 // measured: weights stored in pairs for the packed FMAs (one more load per
 // column) 15.0 ms.
 //
 // The sum over a ray's samples is the reference's (positions entry + k step
 // dir, k < n, binary32 set-up); only its order changes: taps that fall on the
 // same voxel are added as weights first.  The result does not depend on V, on
-// the launch's split of the views or on whether a plane came from shared
-// memory, so every entry point that projects the same rays agrees bit for bit.
+// how a call's views are split into launches (nall), on the slices beside it or
+// on whether a plane came from shared memory.  It does depend on SP, whose parts
+// are summed apart, and so on the call's views, the detector's columns and the SM
+// count: a view by itself can differ in the last bits from the same view in a full
+// call, and the objective's integrals (never split) from the residuals'.
 // Four rays whose columns of a plane do not fit a list (fans steeper than ~65
 // degrees to the sweep axis) add that plane's samples one by one.
 // A column list is shared by four rays, so a voxel that is not finite would

@@ -1,7 +1,8 @@
 // k_slab.cu -- slab-staged forward projection with TMA: cone rays
 // (CUDAmex_FP.cu:56-346) with the OSC forward pass (CUDAmex_oscIter.cu:140-271),
-// general3D rays, and parallel / fan rays onto a decoupled detector whose rows
-// fall between slices.  Other parallel / fan rays stay in a slice: k_rows.cu.
+// general3D rays, and parallel / fan rays of volumes of few slices or small calls
+// (fp_uses_rows) and onto a decoupled detector whose rows fall between slices.
+// Other parallel / fan FPs: k_rows.cu.
 //
 // Why: a ray-per-thread march that fetches its 8 trilinear taps through L1
 // issues ~28 L1 wavefronts per warp-sample, because the 32 rays of a warp
