@@ -80,8 +80,10 @@ static std::mutex g_live_mu;
 static std::vector<mexct_ctx*> g_live;
 static std::atomic<int> g_fail{0};
 
-// Frees the optional buffers of the current device's contexts (those in use by
-// another thread's call keep theirs); whether there were any.
+// Frees the optional buffers of the current device's contexts once all queued work
+// is done (those in use by another thread's call keep theirs; all do where the
+// device cannot be synchronised, as beside another thread's capture); whether there
+// were any.
 static bool give_back() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
@@ -92,8 +94,13 @@ static bool give_back() {
     std::unique_lock<std::recursive_mutex> own(c->mu, std::try_to_lock);
     if (!own.owns_lock()) continue;
     for (Buf* b : c->optional_bufs()) {
-      any |= b->p != nullptr;
+      if (!b->p) continue;
+      if (cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        return any;
+      }
       b->release_synced();
+      any = true;
     }
   }
   return any;
