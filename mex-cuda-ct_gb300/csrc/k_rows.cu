@@ -695,10 +695,14 @@ void fp_rows_shape(int geom, const RayArgs& a, int epi, int sms, int* views, int
 }
 
 // A CTA of the rows kernel works on 128 slices whatever nz is; the slab kernel's
-// work goes with its tiles of eight rows.  A plane of the sweep takes a slab CTA
-// (four per SM) 0.29 us and a rows CTA (two per SM) of 1 / 2 / 4 views 0.80 / 1.33
-// / 2.3 us, so a wave of the rows kernel costs as much as 2.75 / 4.6 / 7.9 waves of
-// the slab kernel (a part-filled last wave counted half full).  Measured, slab ->
+// work goes with its tiles of eight rows (the rows of a last, part-filled tile three
+// quarters of it).  A plane of the sweep takes a wave of slab CTAs (four per SM)
+// 0.29 us and a wave of rows CTAs (two per SM) of 1 / 2 / 4 views 0.75 / 1.36 / 2.0
+// us, and a CTA's fixed work stands for 35 planes (slab) and 45 (four views): the
+// factors below, fitted to 568 pairs of times of W = 64 .. 512 with 30 .. 720 views
+// and 1 .. 128 slices.  The form taken is at most 10 % slower than the other there,
+// and 4 % in all but five.  (The OSC epilogue's stores weigh more on the fewer rows
+// CTAs: 256^2 x 48, 360 / 6 breaks even at ~50 slices, 1.1.)  Measured, slab ->
 // rows at 16, 32, 48, 64 slices: 512^2 x 720 parallel 5.5 -> 11.0, 10.8 -> 11.0,
 // 16.1 -> 11.1, 21.4 -> 11.1 ms (one slice: 1.5 -> 11.0); 128^2 x 180 156 -> 326,
 // 248 -> 328, 348 -> 330, 447 -> 324 us; 512^2 x 90 0.77 -> 1.98, 1.47 -> 1.98, 2.18
@@ -719,9 +723,11 @@ bool fp_uses_rows(int geom, const RayArgs& a, int nz, int epi, int sms) {
   fp_rows_shape(geom, a, epi, sms, &v, &split);
   if (split > 1) return epi == 0 ? tz > 6 : tz > 1 || 4 * bundles <= sms;
   const double wave = (double)((views + v - 1) / v * tiles_u) / (2.0 * sms);
-  const double rows = std::max(1.0, 0.5 * (wave + std::ceil(wave)));
-  const double slab = (double)(bundles * tz) / (4.0 * sms);
-  return slab > rows * (v == 4 ? 7.9 : v == 2 ? 4.6 : 2.75);
+  const double rows = std::max(1.0, 0.1 * wave + 0.9 * std::ceil(wave)) *
+                      (v == 4 ? 6.8 * (1.0 + 45.0 / a.S) : v == 2 ? 4.7 : 2.6) *
+                      (epi == 1 ? 1.1 : 1.0);
+  const double slab = bundles * (0.25 * tz + 0.75 * nz / 8.0) / (4.0 * sms) * (1.0 + 35.0 / a.S);
+  return slab > rows;
 }
 
 int rows_pitch(int nz, int dtype) {
